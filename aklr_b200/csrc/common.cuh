@@ -111,6 +111,26 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// One lane of a converged warp, the same one at every call.  The compiler takes a region under elect.sync's predicate for
+// what it is -- one thread of a warp whose other lanes are at the same place -- and keeps the operands of tcgen05 and TMA
+// instructions in uniform registers.  Under `lane == 0` it cannot: each tcgen05.mma then costs its thread 77-100 cycles
+// instead of 30 (four N = 256 MMAs from an idle pipe: 309 against 132 cycles of issue).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
+// mbar_wait by a whole converged warp; the result is the same in every lane, so the loop around it stays converged.
+template <bool SPIN = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int where) {
+  return __all_sync(0xFFFFFFFFu, mbar_wait<SPIN>(bar, parity, abort_flag, status, where));
+}
+
 // After a wait gave up, one thread of the CTA copies the call's status words to the device's
 // host-visible pair (mapped pinned host memory, or null): the host looks at it at the start of every
 // later call, so a caller that never reads its workspace's status still hears of the failure.

@@ -137,8 +137,9 @@ grouped_gemm_kernel(const __grid_constant__ GroupedGemmParams p) {
   // and the block table that says which expert's they are comes from the sort, which ran before the kernel before
   // this one -- every kernel of the library signals its dependents only after its own wait, so whatever preceded
   // the previous kernel is complete when this one starts.  The activation boxes of those stages follow the wait.
-  int early = 0;  // K-blocks of the first tile whose weight loads are already in flight (producer thread only)
-  if (warp == 0 && lane == 0) {
+  int early = 0;  // K-blocks of the first tile whose weight loads are already in flight (producer warp only)
+  const bool leader = elect_one();
+  if (warp == 0) {
     int nb0 = *p.num_blocks;
     if (nb0 > p.max_blocks) nb0 = p.max_blocks;
     const int tiles_per_block0 = p.out_dim >> kTileShift;
@@ -146,7 +147,7 @@ grouped_gemm_kernel(const __grid_constant__ GroupedGemmParams p) {
       const int b = blockIdx.x / tiles_per_block0, j = blockIdx.x - b * tiles_per_block0;
       const int w_row = p.block_expert[b] * p.rows_per_expert + (j << kTileShift);
       early = KB < S ? KB : S;
-      for (int kb = 0; kb < early; ++kb) {
+      for (int kb = 0; kb < early && leader; ++kb) {
         uint8_t* st = smem + kb * L.stage_bytes;
         mbar_expect_tx(&full[kb], L.stage_bytes);  // the activation box's bytes too: it comes after the wait
         int wx, wy;
@@ -168,21 +169,21 @@ grouped_gemm_kernel(const __grid_constant__ GroupedGemmParams p) {
 
   if (warp == 0) {
     // ------------------------------- TMA producer ------------------------------------------
-    if (lane == 0) {
-      uint32_t it = 0;
-      int s = 0;  // ring position and the parity of its current use
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int b = t / tiles_per_block, j = t - b * tiles_per_block;
-        const int e = p.block_expert[b];
-        const int w_row = e * p.rows_per_expert + (j << kTileShift);
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          uint8_t* st = smem + s * L.stage_bytes;
-          if (static_cast<int>(it) >= early) {  // else: stage free from the start, bytes announced and weights under way
-            bool got;
-            got = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 1);
-            if (!got) { ok = false; break; }
+    // The whole warp walks the loop, one elected lane issues (see elect_one).
+    uint32_t it = 0;
+    int s = 0;  // ring position and the parity of its current use
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      const int b = t / tiles_per_block, j = t - b * tiles_per_block;
+      const int e = p.block_expert[b];
+      const int w_row = e * p.rows_per_expert + (j << kTileShift);
+      for (int kb = 0; kb < KB; ++kb, ++it) {
+        uint8_t* st = smem + s * L.stage_bytes;
+        const bool weights = static_cast<int>(it) >= early;  // else: stage free from the start, bytes announced and weights under way
+        if (weights && !mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, p.status, 1)) { ok = false; break; }
+        if (leader) {
+          if (weights) {
             mbar_expect_tx(&full[s], L.stage_bytes);
             int wx, wy;
             weight_box(p.w_tiled != 0, KB, w_row, kb, &wx, &wy);
@@ -193,30 +194,26 @@ grouped_gemm_kernel(const __grid_constant__ GroupedGemmParams p) {
             }
           }
           tma_load_2d(st + (TWO ? 2 : 1) * kWTileBytes, &p.map_x, &full[s], kb * 128, b * BM);
-          if (++s == S) { s = 0; ph ^= 1; }
         }
+        if (++s == S) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer --------------------------------------------
-    if (lane == 0) {
-      // A lone thread pays the full latency of every instruction: ring position, phases and
-      // descriptors are carried forward, and one commit per K-block serves both the producer (stage
-      // free) and the epilogue (partial complete).
-      int s = 0;
-      uint32_t ph = 0, buf = 0, bph = 0;
-      const uint64_t desc0 = umma_desc_sw128(smem_u32(smem));
-      const uint32_t stage_step = static_cast<uint32_t>(L.stage_bytes) >> 4;
-      uint64_t da0 = desc0;  // first weight tile of stage s; the second one and the token tile follow
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        for (int kb = 0; kb < KB; ++kb) {
-          bool got;
-          got = mbar_wait(&full[s], ph, abort_flag, p.status, 2);
-          if (!got) { ok = false; break; }
-          got = mbar_wait(&tmem_empty[buf], bph ^ 1, abort_flag, p.status, 3);
-          if (!got) { ok = false; break; }
-          tc_fence_after_sync();
+    // Ring position, phases and descriptors are carried forward, and one commit per K-block serves both the producer
+    // (stage free) and the epilogue (partial complete).
+    int s = 0;
+    uint32_t ph = 0, buf = 0, bph = 0;
+    const uint64_t desc0 = umma_desc_sw128(smem_u32(smem));
+    const uint32_t stage_step = static_cast<uint32_t>(L.stage_bytes) >> 4;
+    uint64_t da0 = desc0;  // first weight tile of stage s; the second one and the token tile follow
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 2)) { ok = false; break; }
+        if (!mbar_wait_warp(&tmem_empty[buf], bph ^ 1, abort_flag, p.status, 3)) { ok = false; break; }
+        tc_fence_after_sync();
+        if (leader) {
           const uint64_t da1 = da0 + (kWTileBytes >> 4);
           const uint64_t db = da0 + (((TWO ? 2 : 1) * kWTileBytes) >> 4);
           const uint32_t d = tmem_base + buf * BUF_COLS;
@@ -226,11 +223,11 @@ grouped_gemm_kernel(const __grid_constant__ GroupedGemmParams p) {
             if (TWO) umma_f8f6f4(d + BM, da1 + 2 * k, db + 2 * k, IDESC, k > 0);
           }
           tc_commit(&empty[s]);
-          da0 += stage_step;
-          if (++s == S) { s = 0; ph ^= 1; da0 = desc0; }
-          bph ^= buf;
-          buf ^= 1;
         }
+        da0 += stage_step;
+        if (++s == S) { s = 0; ph ^= 1; da0 = desc0; }
+        bph ^= buf;
+        buf ^= 1;
       }
     }
   } else {

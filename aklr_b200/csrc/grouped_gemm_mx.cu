@@ -229,29 +229,31 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
 
   if (warp == 0) {
     // ------------------------------- TMA producer ------------------------------------------
-    if (lane == 0) {
-      int s = 0;  // ring position and the parity of its current use
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int b = t / tiles_per_block, j = t - b * tiles_per_block;
-        const int e = p.block_expert[b];
-        const int w_row = e * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256);
-        // A decode batch leaves most of a 128-row block as padding (the sort puts the routed rows
-        // first, -1 after them).  Loading all 128 activation rows per K-block made shared-memory
-        // fill traffic from L2, not HBM, the bound (32 KB per K-block against 16 KB of weights): a
-        // block with at most 32 or 64 routed rows loads only those.  The rows left stale feed TMEM
-        // lanes whose results are never stored.
-        const CUtensorMap* map_x = &p.map_x;
-        uint32_t x_bytes = kABytes;
-        if (!SPLIT && p.small_boxes) {
-          const int id32 = p.sorted_ids[b * kBM + 32], id64 = p.sorted_ids[b * kBM + 64];
-          if (id32 < 0) { map_x = &p.map_x_rows32; x_bytes = 32 * 128; }
-          else if (id64 < 0) { map_x = &p.map_x_rows64; x_bytes = 64 * 128; }
-        }
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 21)) { ok = false; break; }
-          uint8_t* st = smem + s * kStageBytes;
+    // The whole warp walks the loop, one elected lane issues (see elect_one).
+    const bool leader = elect_one();
+    int s = 0;  // ring position and the parity of its current use
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      const int b = t / tiles_per_block, j = t - b * tiles_per_block;
+      const int e = p.block_expert[b];
+      const int w_row = e * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256);
+      // A decode batch leaves most of a 128-row block as padding (the sort puts the routed rows
+      // first, -1 after them).  Loading all 128 activation rows per K-block made shared-memory
+      // fill traffic from L2, not HBM, the bound (32 KB per K-block against 16 KB of weights): a
+      // block with at most 32 or 64 routed rows loads only those.  The rows left stale feed TMEM
+      // lanes whose results are never stored.
+      const CUtensorMap* map_x = &p.map_x;
+      uint32_t x_bytes = kABytes;
+      if (!SPLIT && p.small_boxes) {
+        const int id32 = p.sorted_ids[b * kBM + 32], id64 = p.sorted_ids[b * kBM + 64];
+        if (id32 < 0) { map_x = &p.map_x_rows32; x_bytes = 32 * 128; }
+        else if (id64 < 0) { map_x = &p.map_x_rows64; x_bytes = 64 * 128; }
+      }
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, p.status, 21)) { ok = false; break; }
+        uint8_t* st = smem + s * kStageBytes;
+        if (leader) {
           // the transaction count of the unpacking fp4 load is its packed size (what crosses from
           // global memory), not the padded bytes it writes: expecting the padded size never completes
           mbar_expect_tx(&full[s], (SPLIT ? 2 : 1) * x_bytes + kBBytes / 2);
@@ -263,34 +265,30 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
           } else {
             tma_load_2d(st + kOffB, &p.map_w, &full[s], kb * 128, w_row);
           }
-          if (++s == S) { s = 0; ph ^= 1; }
         }
+        if (++s == S) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer --------------------------------------------
-    if (lane == 0) {
-      // A lone thread pays the full latency of every instruction: ring position, phase and the
-      // five descriptors are carried forward, not recomputed.
-      uint32_t it = 0, tile_no = 0;
-      int s = 0;
-      uint32_t ph = 0;
-      const uint32_t base = smem_u32(smem);
-      const uint64_t da0 = umma_desc_sw128(base), db0 = umma_desc_sw128(base + kOffB);
-      const uint64_t sfa0 = sf_desc(base + kOffSf);
-      uint32_t step = 0;  // (stage * kStageBytes) >> 4, added to the address field of each descriptor
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_no) {
-        // the single accumulator must have been read out by the previous tile's epilogue
-        bool got;
-        got = mbar_wait(acc_empty, (tile_no & 1) ^ 1, abort_flag, p.status, 22);
-        if (!got) break;
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          got = mbar_wait(&full[s], ph, abort_flag, p.status, 23);
-          if (!got) { ok = false; break; }
-          got = mbar_wait(&sf_full[s], ph, abort_flag, p.status, 24);
-          if (!got) { ok = false; break; }
-          tc_fence_after_sync();
+    // Ring position, phase and the five descriptors are carried forward, not recomputed.
+    const bool leader = elect_one();
+    uint32_t tile_no = 0;
+    int s = 0;
+    uint32_t ph = 0;
+    const uint32_t base = smem_u32(smem);
+    const uint64_t da0 = umma_desc_sw128(base), db0 = umma_desc_sw128(base + kOffB);
+    const uint64_t sfa0 = sf_desc(base + kOffSf);
+    uint32_t step = 0;  // (stage * kStageBytes) >> 4, added to the address field of each descriptor
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_no) {
+      // the single accumulator must have been read out by the previous tile's epilogue
+      if (!mbar_wait_warp(acc_empty, (tile_no & 1) ^ 1, abort_flag, p.status, 22)) break;
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 23)) { ok = false; break; }
+        if (!mbar_wait_warp(&sf_full[s], ph, abort_flag, p.status, 24)) { ok = false; break; }
+        tc_fence_after_sync();
+        if (leader) {
           const uint64_t sfa = sfa0 + step;
           tmem_cp_32x128b_warpx4(tmem_base + kSfaCol, sfa);
           tmem_cp_32x128b_warpx4(tmem_base + kSfbCol, sfa + (kSfaBytes >> 4));
@@ -306,11 +304,11 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
                       tmem_base + kSfbCol, 1u);
           }
           tc_commit(&empty[s]);
-          step += kStageBytes >> 4;
-          if (++s == S) { s = 0; ph ^= 1; step = 0; }
         }
-        if (ok) tc_commit(acc_full);
+        step += kStageBytes >> 4;
+        if (++s == S) { s = 0; ph ^= 1; step = 0; }
       }
+      if (ok && leader) tc_commit(acc_full);
     }
   } else if (warp >= 10) {
     // ------------------- scale-factor staging, running ahead of the MMA warp -------------------

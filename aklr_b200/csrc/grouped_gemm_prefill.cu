@@ -179,20 +179,22 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_prefill_kernel(const
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsLean));
   if (warp == 0) {
     // ------------------------------- TMA producer ------------------------------------------
-    if (lane == 0) {
-      int s = 0;        // ring position and the parity of its current use
-      uint32_t ph = 0;
-      bool ok = true;
-      const uint32_t full0 = PAIR ? mapa_shared(smem_u32(full), 0) : 0u;  // the even CTA's "full" barriers
-      for (int t = worker; t < total_tiles && ok; t += n_workers) {
-        const int u = t / tiles_per_block, j = t - u * tiles_per_block;
-        bool live;
-        const int b = block_of(u, &live);
-        const int e = p.block_expert[b];
-        const int w_row = e * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256);
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!mbar_wait<PAIR>(&empty[s], ph ^ 1, abort_flag, p.status, 11)) { ok = false; break; }
-          uint8_t* st = smem + s * kStageBytes;
+    // The whole warp walks the loop, one elected lane issues (see elect_one).
+    const bool leader = elect_one();
+    int s = 0;        // ring position and the parity of its current use
+    uint32_t ph = 0;
+    bool ok = true;
+    const uint32_t full0 = PAIR ? mapa_shared(smem_u32(full), 0) : 0u;  // the even CTA's "full" barriers
+    for (int t = worker; t < total_tiles && ok; t += n_workers) {
+      const int u = t / tiles_per_block, j = t - u * tiles_per_block;
+      bool live;
+      const int b = block_of(u, &live);
+      const int e = p.block_expert[b];
+      const int w_row = e * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256);
+      for (int kb = 0; kb < KB; ++kb) {
+        if (!mbar_wait_warp<PAIR>(&empty[s], ph ^ 1, abort_flag, p.status, 11)) { ok = false; break; }
+        uint8_t* st = smem + s * kStageBytes;
+        if (leader) {
           if (PAIR) {
             if (rank == 0) mbar_expect_tx(&full[s], 2 * kStageBytes);  // both CTAs' bytes
             const uint32_t bar = full0 + s * 8;
@@ -217,43 +219,39 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_prefill_kernel(const
               tma_load_2d(st + kABytes, &p.map_w, &full[s], kb * 128, w_row);  // box of 256 rows
             }
           }
-          if (++s == S) { s = 0; ph ^= 1; }
         }
+        if (++s == S) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issuer --------------------------------------------
-    if (lane == 0 && rank == 0) {
-      // This thread is alone in its warp, so every instruction here costs its full latency:
-      // the loop carries ring positions and descriptors forward instead of recomputing them.
-      uint32_t it = 0;
+    if (rank == 0) {
+      // The loop carries ring positions and descriptors forward instead of recomputing them.
+      const bool leader = elect_one();
       int s = 0;
       uint32_t ph = 0, buf = 0, bph = 0;
       const uint64_t desc0 = umma_desc_sw128(smem_u32(smem));
       uint64_t da = desc0;  // descriptor of stage s' token tile; the weight tile follows it
       bool ok = true;
       for (int t = worker; t < total_tiles && ok; t += n_workers) {
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          bool got;
-          got = mbar_wait<PAIR>(&full[s], ph, abort_flag, p.status, 12);
-          if (!got) { ok = false; break; }
+        for (int kb = 0; kb < KB; ++kb) {
+          if (!mbar_wait_warp<PAIR>(&full[s], ph, abort_flag, p.status, 12)) { ok = false; break; }
           // One N=256 MMA per 32 K bytes into this K-block's TMEM buffer and a single commit per
           // K-block: the barrier that frees the shared-memory stage also tells the epilogue that
-          // the partial is complete.  (Two N=128 groups with their own hand-offs, so that the
-          // epilogue could start on the first half earlier, measured 20% slower: every extra commit
-          // and barrier round costs more than the overlap gains.)
-          got = mbar_wait<PAIR>(&tmem_empty[buf], bph ^ 1, abort_flag, p.status, 13);
-          if (!got) { ok = false; break; }
+          // the partial is complete.
+          if (!mbar_wait_warp<PAIR>(&tmem_empty[buf], bph ^ 1, abort_flag, p.status, 13)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint64_t db = da + (kABytes >> 4);
-          const uint32_t d = tmem_base + buf * 256;
+          if (leader) {
+            const uint64_t db = da + (kABytes >> 4);
+            const uint32_t d = tmem_base + buf * 256;
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (PAIR) umma_f8f6f4_pair(d, da + 2 * k, db + 2 * k, umma_idesc_e4m3(256, 256), k > 0);
-            else umma_f8f6f4(d, da + 2 * k, db + 2 * k, umma_idesc_e4m3(256), k > 0);
+            for (int k = 0; k < 4; ++k) {
+              if (PAIR) umma_f8f6f4_pair(d, da + 2 * k, db + 2 * k, umma_idesc_e4m3(256, 256), k > 0);
+              else umma_f8f6f4(d, da + 2 * k, db + 2 * k, umma_idesc_e4m3(256), k > 0);
+            }
+            if (PAIR) tc_commit_pair(&empty[s], 3);
+            else tc_commit(&empty[s]);
           }
-          if (PAIR) tc_commit_pair(&empty[s], 3);
-          else tc_commit(&empty[s]);
           da += kStageBytes >> 4;
           if (++s == S) { s = 0; ph ^= 1; da = desc0; }
           bph ^= buf;

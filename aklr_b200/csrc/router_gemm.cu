@@ -77,34 +77,36 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   const uint32_t tmem_base = *tmem_ptr;
 
   if (warp == 0) {
-    if (lane == 0) {
-      for (int it = 0; it < k_steps; ++it) {
-        const int s = it % kStages;
-        if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, status, 31)) break;
-        uint8_t* st = smem + s * stage_bytes;
+    const bool leader = elect_one();
+    for (int it = 0; it < k_steps; ++it) {
+      const int s = it % kStages;
+      if (!mbar_wait_warp(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, status, 31)) break;
+      uint8_t* st = smem + s * stage_bytes;
+      if (leader) {
         mbar_expect_tx(&full[s], stage_bytes);
         tma_load_2d(st, &p.map_x, &full[s], it * 64, tok0);
         tma_load_2d(st + kABytes, &p.map_w, &full[s], it * 64, exp0);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // kind::f16: f32 accumulator, bf16 A and B, K-major, M 128, N n_tile
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.n_tile >> 3) << 17) |
-                             (static_cast<uint32_t>(128 >> 4) << 24);
-      bool ok = true;
-      for (int it = 0; it < k_steps; ++it) {
-        const int s = it % kStages;
-        if (!mbar_wait(&full[s], (it / kStages) & 1, abort_flag, status, 32)) { ok = false; break; }
-        tc_fence_after_sync();
+    const bool leader = elect_one();
+    // kind::f16: f32 accumulator, bf16 A and B, K-major, M 128, N n_tile
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.n_tile >> 3) << 17) |
+                           (static_cast<uint32_t>(128 >> 4) << 24);
+    bool ok = true;
+    for (int it = 0; it < k_steps; ++it) {
+      const int s = it % kStages;
+      if (!mbar_wait_warp(&full[s], (it / kStages) & 1, abort_flag, status, 32)) { ok = false; break; }
+      tc_fence_after_sync();
+      if (leader) {
         const uint32_t a0 = smem_u32(smem + s * stage_bytes);
         const uint64_t da = umma_desc_sw128(a0), db = umma_desc_sw128(a0 + kABytes);
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(&empty[s]);
       }
-      if (ok) tc_commit(acc_full);
     }
+    if (ok && leader) tc_commit(acc_full);
   } else {
     const int quarter = warp & 3;
     const int token = tok0 + quarter * 32 + lane;
