@@ -331,6 +331,7 @@ int run_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l, co
   ap.block_expert = block_expert;
   ap.counts = reinterpret_cast<int32_t*>(ws + l.counts);
   ap.num_blocks = num_blocks;
+  ap.status = status;
   ap.chunk_hist = reinterpret_cast<int32_t*>(ws + l.chunk_hist);
   ap.n_routes = routes;
   ap.n_experts = experts;
@@ -509,6 +510,7 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
   ap.block_expert = block_expert;
   ap.counts = reinterpret_cast<int32_t*>(ws + l.counts);
   ap.num_blocks = num_blocks;
+  ap.status = status;
   ap.chunk_hist = reinterpret_cast<int32_t*>(ws + l.chunk_hist);
   ap.n_routes = routes;
   ap.n_experts = experts;
@@ -694,8 +696,10 @@ int prepare(const aklr_moe_config* cfg, aklr_moe_workspace_layout* l, void* work
                 static_cast<long long>(l->total_bytes));
   if (reinterpret_cast<uintptr_t>(workspace) % 1024 != 0)
     return fail(AKLR_ERR_BAD_ARGUMENT, "workspace must be 1024-byte aligned");
-  const cudaError_t err = cudaMemsetAsync(static_cast<uint8_t*>(workspace) + l->status, 0, 32, stream);
-  if (err != cudaSuccess) return cuda_fail(err, "clearing the status words");
+  if (cfg->n_tokens == 0) {  // no sort runs that would clear the status words
+    const cudaError_t err = cudaMemsetAsync(static_cast<uint8_t*>(workspace) + l->status, 0, 32, stream);
+    if (err != cudaSuccess) return cuda_fail(err, "clearing the status words");
+  }
   return AKLR_OK;
 }
 
@@ -1179,8 +1183,7 @@ int aklr_router_gemm_bf16(const void* x, const void* w, void* logits, int32_t n_
   // 64 tokens and up: tensor cores (128-token tiles); fewer: the warp-per-dot-product kernel, which
   // spreads the router weight over many SMs
   if (n_tokens >= 64 && hidden % 64 == 0 && n_routed >= 1) {
-    int n_tile = (n_routed + 15) / 16 * 16;
-    if (n_tile > 256) n_tile = 256;
+    const int n_tile = aklr::router_gemm_tc_pick_n_tile(n_tokens, n_routed, sm_count());
     CUtensorMap map_x, map_w;
     rc = make_map_bf16(&map_x, x, n_tokens, hidden, 128);
     if (rc) return rc;

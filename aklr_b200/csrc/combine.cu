@@ -78,49 +78,70 @@ int launch_combine(const CombineParams& p, cudaStream_t stream) {
   return launch_kernel(combine_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
-// One warp per (token, kRouterExperts experts): lanes stride the hidden dimension with 16-byte loads.
-template <int kRouterExperts>
+// One warp per (TOKENS tokens, EXPERTS experts): lanes stride the hidden dimension with 16-byte loads, and the loads of
+// UNROLL strides are on their way before the first product.  What bounds it is the latency of those loads -- a decode
+// call finds the router weight in HBM -- so a warp has 12-16 of them in flight; with the loads of one stride at a time
+// (28 strides at 7168) one token on 256 experts took 16.9 us and 17 tokens on 2048 x 512 31 us.  Several tokens per warp
+// share a weight load and several experts a token load.  Each dot product is the same chain of FMAs whatever the shape.
+template <int TOKENS, int EXPERTS, int UNROLL>
 __global__ void __launch_bounds__(256)
 router_gemm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ logits,
                    int n_tokens, int hidden, int n_routed) {
   const int lane = threadIdx.x & 31;
-  const int groups = (n_routed + kRouterExperts - 1) / kRouterExperts;
-  const int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (item >= static_cast<int64_t>(n_tokens) * groups) return;
-  const int token = static_cast<int>(item / groups);
-  const int e0 = static_cast<int>(item - static_cast<int64_t>(token) * groups) * kRouterExperts;
-  float acc[kRouterExperts];
+  const int groups = (n_routed + EXPERTS - 1) / EXPERTS;
+  const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int tok0 = item / groups * TOKENS, e0 = item % groups * EXPERTS;
+  griddep_wait();
+  griddep_launch();
+  if (tok0 >= n_tokens) return;
+  const uint16_t* xp[TOKENS];  // rows past the end repeat the last one and are not stored
+  const uint16_t* wp[EXPERTS];
 #pragma unroll
-  for (int j = 0; j < kRouterExperts; ++j) acc[j] = 0.0f;
-  for (int h = lane * 8; h < hidden; h += 256) {
-    const uint4 xr = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(token) * hidden + h);
-    const uint32_t xw[4] = {xr.x, xr.y, xr.z, xr.w};
+  for (int t = 0; t < TOKENS; ++t) xp[t] = x + static_cast<size_t>(min(tok0 + t, n_tokens - 1)) * hidden;
 #pragma unroll
-    for (int j = 0; j < kRouterExperts; ++j) {
-      if (e0 + j < n_routed) {
-        const uint4 wr = *reinterpret_cast<const uint4*>(w + static_cast<size_t>(e0 + j) * hidden + h);
-        const uint32_t ww[4] = {wr.x, wr.y, wr.z, wr.w};
+  for (int j = 0; j < EXPERTS; ++j) wp[j] = w + static_cast<size_t>(min(e0 + j, n_routed - 1)) * hidden;
+  float acc[TOKENS][EXPERTS] = {};
+  for (int h0 = lane * 8; h0 < hidden; h0 += 256 * UNROLL) {
+    uint4 xr[UNROLL][TOKENS], wr[UNROLL][EXPERTS];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          acc[j] = fmaf(__uint_as_float(xw[q] << 16), __uint_as_float(ww[q] << 16), acc[j]);
-          acc[j] = fmaf(__uint_as_float(xw[q] & 0xFFFF0000u), __uint_as_float(ww[q] & 0xFFFF0000u), acc[j]);
+    for (int u = 0; u < UNROLL; ++u) {
+      const int h = h0 + u * 256;
+      if (h < hidden) {
+#pragma unroll
+        for (int j = 0; j < EXPERTS; ++j) wr[u][j] = __ldg(reinterpret_cast<const uint4*>(wp[j] + h));
+#pragma unroll
+        for (int t = 0; t < TOKENS; ++t) xr[u][t] = *reinterpret_cast<const uint4*>(xp[t] + h);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      if (h0 + u * 256 >= hidden) continue;
+#pragma unroll
+      for (int t = 0; t < TOKENS; ++t) {
+        const uint32_t xw[4] = {xr[u][t].x, xr[u][t].y, xr[u][t].z, xr[u][t].w};
+#pragma unroll
+        for (int j = 0; j < EXPERTS; ++j) {
+          const uint32_t ww[4] = {wr[u][j].x, wr[u][j].y, wr[u][j].z, wr[u][j].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[t][j] = fmaf(__uint_as_float(xw[q] << 16), __uint_as_float(ww[q] << 16), acc[t][j]);
+            acc[t][j] = fmaf(__uint_as_float(xw[q] & 0xFFFF0000u), __uint_as_float(ww[q] & 0xFFFF0000u), acc[t][j]);
+          }
         }
       }
     }
   }
 #pragma unroll
-  for (int j = 0; j < kRouterExperts; ++j) {
+  for (int t = 0; t < TOKENS; ++t)
 #pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) acc[j] += __shfl_xor_sync(0xFFFFFFFFu, acc[j], off);
-  }
-  if (lane < kRouterExperts && e0 + lane < n_routed) {
-    float v = acc[0];
+    for (int j = 0; j < EXPERTS; ++j) {
 #pragma unroll
-    for (int j = 1; j < kRouterExperts; ++j)
-      if (lane == j) v = acc[j];
-    const __nv_bfloat16 r = __float2bfloat16_rn(v);
-    logits[static_cast<size_t>(token) * n_routed + e0 + lane] = *reinterpret_cast<const uint16_t*>(&r);
-  }
+      for (int off = 16; off >= 1; off >>= 1) acc[t][j] += __shfl_xor_sync(0xFFFFFFFFu, acc[t][j], off);
+      if (lane == t * EXPERTS + j && tok0 + t < n_tokens && e0 + j < n_routed) {
+        const __nv_bfloat16 r = __float2bfloat16_rn(acc[t][j]);
+        logits[static_cast<size_t>(tok0 + t) * n_routed + e0 + j] = *reinterpret_cast<const uint16_t*>(&r);
+      }
+    }
 }
 
 // Qwen2-MoE's gated shared expert (aklr/plugins/sglang/models/qwen2_moe/reference.py:84-90): the
@@ -258,18 +279,31 @@ int launch_add_gated_rows(const void* x, const void* gate, const void* rows, voi
 __global__ void __launch_bounds__(256)
 router_dot_f32_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,
                       int n_tokens, int hidden, int n_routed) {
+  constexpr int UNROLL = 8;  // strides whose loads are in flight together (see router_gemm_kernel)
   const int lane = threadIdx.x & 31;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  griddep_wait();
+  griddep_launch();
   if (item >= static_cast<int64_t>(n_tokens) * n_routed) return;
   const int token = static_cast<int>(item / n_routed), e = static_cast<int>(item - static_cast<int64_t>(token) * n_routed);
   float acc = 0.0f;
-  for (int h = lane * 4; h < hidden; h += 128) {
-    const uint2 xr = *reinterpret_cast<const uint2*>(x + static_cast<size_t>(token) * hidden + h);
-    const float4 wr = *reinterpret_cast<const float4*>(w + static_cast<size_t>(e) * hidden + h);
-    acc = fmaf(__uint_as_float(xr.x << 16), wr.x, acc);
-    acc = fmaf(__uint_as_float(xr.x & 0xFFFF0000u), wr.y, acc);
-    acc = fmaf(__uint_as_float(xr.y << 16), wr.z, acc);
-    acc = fmaf(__uint_as_float(xr.y & 0xFFFF0000u), wr.w, acc);
+  for (int h0 = lane * 4; h0 < hidden; h0 += 128 * UNROLL) {
+    uint2 xr[UNROLL];
+    float4 wr[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (h0 + u * 128 < hidden) {
+        wr[u] = __ldg(reinterpret_cast<const float4*>(w + static_cast<size_t>(e) * hidden + h0 + u * 128));
+        xr[u] = *reinterpret_cast<const uint2*>(x + static_cast<size_t>(token) * hidden + h0 + u * 128);
+      }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      if (h0 + u * 128 < hidden) {
+        acc = fmaf(__uint_as_float(xr[u].x << 16), wr[u].x, acc);
+        acc = fmaf(__uint_as_float(xr[u].x & 0xFFFF0000u), wr[u].y, acc);
+        acc = fmaf(__uint_as_float(xr[u].y << 16), wr[u].z, acc);
+        acc = fmaf(__uint_as_float(xr[u].y & 0xFFFF0000u), wr[u].w, acc);
+      }
   }
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
@@ -286,6 +320,8 @@ router_tile_f32_kernel(const uint16_t* __restrict__ x, const float* __restrict__
   const int token0 = blockIdx.x * BM, e0 = blockIdx.y * BN;
   const int lrow = tid >> 2, lk = (tid & 3) * 4;  // this thread stages 4 k of one row of each tile
   float acc[4][4] = {};
+  griddep_wait();
+  griddep_launch();
   for (int k0 = 0; k0 < hidden; k0 += BK) {
     uint2 xr = make_uint2(0u, 0u);
     float4 wr = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -331,32 +367,33 @@ int launch_router_gemm_f32(const void* x, const float* w, float* logits, int n_t
   auto* xp = static_cast<const uint16_t*>(x);
   if (n_tokens <= 16) {
     const int64_t blocks = (static_cast<int64_t>(n_tokens) * n_routed + 7) / 8;
-    router_dot_f32_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(xp, w, logits, n_tokens, hidden, n_routed);
-  } else {
-    const dim3 grid((n_tokens + 63) / 64, (n_routed + 63) / 64);
-    router_tile_f32_kernel<<<grid, 256, 0, stream>>>(xp, w, logits, n_tokens, hidden, n_routed);
+    return launch_kernel(router_dot_f32_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, 1, xp, w, logits, n_tokens,
+                         hidden, n_routed) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
   }
-  return cudaGetLastError() == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  const dim3 grid((n_tokens + 63) / 64, (n_routed + 63) / 64);
+  return launch_kernel(router_tile_f32_kernel, grid, dim3(256), 0, stream, 1, xp, w, logits, n_tokens, hidden, n_routed) == cudaSuccess
+             ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 int launch_router_gemm(const void* x, const void* w, void* logits, int n_tokens, int hidden, int n_routed,
                        cudaStream_t stream) {
   if (hidden % 8 != 0) return AKLR_ERR_UNSUPPORTED_SHAPE;
   if (n_tokens == 0) return AKLR_OK;
-  // few tokens: one expert per warp so the router weight is streamed by many SMs
-  const int per_warp = n_tokens <= 16 ? 1 : 8;
-  const int groups = (n_routed + per_warp - 1) / per_warp;
-  const int64_t items = static_cast<int64_t>(n_tokens) * groups;
-  const int64_t blocks = (items + 7) / 8;
-  if (blocks > 0x7FFFFFFF) return AKLR_ERR_TOO_LARGE;
   auto* xp = static_cast<const uint16_t*>(x);
   auto* wp = static_cast<const uint16_t*>(w);
   auto* lp = static_cast<uint16_t*>(logits);
-  if (per_warp == 1)
-    router_gemm_kernel<1><<<static_cast<int>(blocks), 256, 0, stream>>>(xp, wp, lp, n_tokens, hidden, n_routed);
-  else
-    router_gemm_kernel<8><<<static_cast<int>(blocks), 256, 0, stream>>>(xp, wp, lp, n_tokens, hidden, n_routed);
-  return cudaGetLastError() == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  auto run = [&](auto kernel, int tokens, int experts, int warps) {
+    const int64_t items = static_cast<int64_t>((n_tokens + tokens - 1) / tokens) * ((n_routed + experts - 1) / experts);
+    const int64_t blocks = (items + warps - 1) / warps;
+    if (items > 0x7FFFFFFF - 32) return AKLR_ERR_TOO_LARGE;
+    return launch_kernel(kernel, dim3(static_cast<unsigned>(blocks)), dim3(32 * warps), 0, stream, 1, xp, wp, lp, n_tokens, hidden,
+                         n_routed) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  };
+  // One token: one dot product per warp and two warps per CTA, so that the weight is read by every SM.  More tokens
+  // reuse what a warp has loaded: at 17 tokens on 2048 x 512 2 x 4 products per warp read 27 MB from L2, 1 x 8 35 MB.
+  if (n_tokens == 1) return run(router_gemm_kernel<1, 1, 8>, 1, 1, 2);
+  if (n_tokens <= 16) return run(router_gemm_kernel<2, 2, 4>, 2, 2, 4);
+  return run(router_gemm_kernel<2, 4, 2>, 2, 4, 8);
 }
 
 }  // namespace aklr

@@ -37,6 +37,7 @@ struct AlignParams {
   int32_t* block_expert;      // [max_blocks]
   int32_t* counts;            // [n_experts]
   int32_t* num_blocks;        // [2]: blocks used, rows used (= blocks * block_m); [3] with pair_table: + pairs
+  int32_t* status;            // optional [2]: the call's status words, cleared by the sort
   int32_t* pair_table;        // optional [max_blocks]: first block of every run of <= 2 blocks of one
                               // expert; bit 31 set when the second block exists
   int32_t* chunk_hist;        // [ceil(n_routes/1024) * n_experts] scratch
@@ -245,6 +246,7 @@ struct EpCombineParams {
 int launch_ep_combine(const EpCombineParams& p, cudaStream_t stream);
 
 // tensor-core router GEMM (router_gemm.cu): maps are bf16 [T,H] box 64 x 128 and [E,H] box 64 x n_tile
+int router_gemm_tc_pick_n_tile(int n_tokens, int n_routed, int sm_count);
 int launch_router_gemm_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, void* logits, int n_tokens, int hidden,
                           int n_routed, int n_tile, int32_t* host_status, cudaStream_t stream);
 

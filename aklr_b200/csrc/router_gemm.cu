@@ -1,9 +1,15 @@
 // Router projection on the tensor cores, sm_100a: logits[T, E] = bf16( x[T, H] . W[E, H]^T ) with
 // float32 accumulation in TMEM, the rounding point of the reference's _router_logits
-// (aklr/plugins/sglang/models/qwen3_moe/reference.py:24-31).  One CTA per 128 tokens x up to 256
-// experts: TMA (SWIZZLE_128B, 64 bf16 = 128 bytes of K per stage) feeds tcgen05.mma kind::f16
-// (M128, N = experts rounded up to 16, K16); rows and experts past the end are zero-filled by the
+// (aklr/plugins/sglang/models/qwen3_moe/reference.py:24-31).  One CTA per 128 tokens x 16..256
+// experts: TMA (SWIZZLE_128B, 64 bf16 = 128 bytes of K per stage) feeds
+// tcgen05.mma kind::f16 (M128, N = experts of the tile, K16); rows and experts past the end are zero-filled by the
 // TMA.  192 threads: warp 0 TMA, warp 1 MMA + TMEM, warps 2..5 epilogue (one TMEM lane quarter each).
+//
+// A tile's time is the latency of its loads, not their bytes or its arithmetic: with one CTA per 128 tokens and all
+// experts (four stages of 48 KB) 64 tokens on 7168 x 256 took 43 us on ONE SM.  So the experts are spread over as
+// many CTAs as the chip has SMs, which makes the stages small and the ring deep; every logit is still one
+// accumulation over K in the same order, so no bit of it changes (splitting K over CTAs would be faster still and
+// change roundings, and with them picks).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -12,8 +18,9 @@ namespace aklr {
 namespace {
 
 constexpr int kThreads = 192;
-constexpr int kStages = 4;
+constexpr int kMaxStages = 10;
 constexpr int kABytes = 128 * 128;
+constexpr int kSmemBudget = 222 * 1024;  // stages; barriers and alignment slack fit in the rest of 227 KB
 
 struct RouterParams {
   CUtensorMap map_x;  // bf16 [T, H], box 64 x 128
@@ -21,7 +28,7 @@ struct RouterParams {
   uint16_t* logits;   // bf16 [T, E]
   int32_t* status;    // optional [2]
   int32_t* host_status;  // the device's host-visible copy of a failure (or null)
-  int n_tokens, hidden, n_routed, n_tile;
+  int n_tokens, hidden, n_routed, n_tile, stages;
 };
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
@@ -38,6 +45,7 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stage_bytes = kABytes + p.n_tile * 128;
+  const int kStages = p.stages;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * stage_bytes);
   uint64_t* empty = full + kStages;
   uint64_t* acc_full = empty + kStages;
@@ -75,18 +83,22 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr;
+  griddep_wait();
+  griddep_launch();
 
   if (warp == 0) {
     const bool leader = elect_one();
+    int s = 0;
+    uint32_t ph = 0;
     for (int it = 0; it < k_steps; ++it) {
-      const int s = it % kStages;
-      if (!mbar_wait_warp(&empty[s], ((it / kStages) & 1) ^ 1, abort_flag, status, 31)) break;
+      if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, status, 31)) break;
       uint8_t* st = smem + s * stage_bytes;
       if (leader) {
         mbar_expect_tx(&full[s], stage_bytes);
         tma_load_2d(st, &p.map_x, &full[s], it * 64, tok0);
         tma_load_2d(st + kABytes, &p.map_w, &full[s], it * 64, exp0);
       }
+      if (++s == kStages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
@@ -94,9 +106,10 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.n_tile >> 3) << 17) |
                            (static_cast<uint32_t>(128 >> 4) << 24);
     bool ok = true;
+    int s = 0;
+    uint32_t ph = 0;
     for (int it = 0; it < k_steps; ++it) {
-      const int s = it % kStages;
-      if (!mbar_wait_warp(&full[s], (it / kStages) & 1, abort_flag, status, 32)) { ok = false; break; }
+      if (!mbar_wait_warp(&full[s], ph, abort_flag, status, 32)) { ok = false; break; }
       tc_fence_after_sync();
       if (leader) {
         const uint32_t a0 = smem_u32(smem + s * stage_bytes);
@@ -105,6 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
         for (int k = 0; k < 4; ++k) umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(&empty[s]);
       }
+      if (++s == kStages) { s = 0; ph ^= 1; }
     }
     if (ok && leader) tc_commit(acc_full);
   } else {
@@ -154,6 +168,15 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
 
 }  // namespace
 
+// Experts per CTA: the fewest (a power of two from 16, what the layout of the logits allows to be written in whole
+// sectors) whose CTAs still fit the chip in one wave.
+int router_gemm_tc_pick_n_tile(int n_tokens, int n_routed, int sm_count) {
+  const int64_t token_tiles = (n_tokens + 127) / 128;
+  int n_tile = 16;
+  while (n_tile < 256 && n_tile < n_routed && token_tiles * ((n_routed + n_tile - 1) / n_tile) > sm_count) n_tile *= 2;
+  return n_tile;
+}
+
 int launch_router_gemm_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, void* logits, int n_tokens, int hidden,
                           int n_routed, int n_tile, int32_t* host_status, cudaStream_t stream) {
   if (hidden % 64 != 0 || n_tile % 16 != 0 || n_tile < 16 || n_tile > 256) return AKLR_ERR_UNSUPPORTED_SHAPE;
@@ -167,11 +190,12 @@ int launch_router_gemm_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, vo
   p.hidden = hidden;
   p.n_routed = n_routed;
   p.n_tile = n_tile;
-  const size_t smem = static_cast<size_t>(kStages) * (kABytes + n_tile * 128) + (2 * kStages + 1) * 8 + 32 + 1024;
+  p.stages = kSmemBudget / (kABytes + n_tile * 128);
+  if (p.stages > kMaxStages) p.stages = kMaxStages;
+  const size_t smem = static_cast<size_t>(p.stages) * (kABytes + n_tile * 128) + (2 * p.stages + 1) * 8 + 32 + 1024;
   if (ensure_max_dynamic_smem(reinterpret_cast<const void*>(router_gemm_tc_kernel)) != AKLR_OK) return AKLR_ERR_CUDA;
   const dim3 grid((n_tokens + 127) / 128, (n_routed + n_tile - 1) / n_tile);
-  router_gemm_tc_kernel<<<grid, kThreads, smem, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  return launch_kernel(router_gemm_tc_kernel, grid, dim3(kThreads), smem, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 }  // namespace aklr

@@ -439,6 +439,9 @@ __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, i
   if (tid == nt - 1) {
     p.num_blocks[0] = all_blocks;
     p.num_blocks[1] = all_blocks * p.block_m;
+    // Cleared here and not by a memset of the call's own: a memset node between the router's kernel and the routing
+    // is 4-5 us of a decode call (1.5 us of its own and a launch gap on either side, no programmatic overlap).
+    if (p.status) p.status[0] = p.status[1] = 0;
   }
   int pair_running = 0;  // runs of <= 2 blocks before this thread's experts
   if (p.pair_table) {
