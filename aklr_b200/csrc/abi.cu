@@ -541,7 +541,7 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
   if (split && fp4) return fail(AKLR_ERR_BAD_ARGUMENT, "activations are kept in bf16 or quantised to MXFP4, not both");
   if (fp4 && q_in) return fail(AKLR_ERR_BAD_ARGUMENT, "rows that arrive quantised are MXFP8");
   qp.act_fp4 = fp4;
-  qp.zero_padding = small_activation_boxes(c) && !split ? 2 : 1;
+  qp.zero_padding = small_activation_boxes(c) ? 2 : 1;
   const int64_t cap = l.capacity;
   uint8_t* xq_lo = ws + l.xq + align_up(cap * c.hidden, 1024);
   uint8_t* xs_lo = ws + l.xs + align_up(cap * (c.hidden / 128) * 4, 256);
@@ -583,16 +583,20 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
   if (rc) return rc;
   rc = make_map_u8(&g1.map_x, ws + l.xq, l.capacity, c.hidden, 128);
   if (rc) return rc;
-  rc = make_map_u8(&g1.map_x_rows32, ws + l.xq, l.capacity, c.hidden, 32);
-  if (rc) return rc;
-  rc = make_map_u8(&g1.map_x_rows64, ws + l.xq, l.capacity, c.hidden, 64);
-  if (rc) return rc;
-  g1.small_boxes = small_activation_boxes(c) && !split;
+  g1.small_boxes = small_activation_boxes(c);
+  for (int i = 0; i < 3 && g1.small_boxes; ++i) {
+    rc = make_map_u8(&g1.map_x_small[i], ws + l.xq, l.capacity, c.hidden, 16 << i);
+    if (rc) return rc;
+  }
   g1.split = split;
   g1.act_fp4 = fp4;
   if (split) {
     rc = make_map_u8(&g1.map_x_lo, xq_lo, l.capacity, c.hidden, 128);
     if (rc) return rc;
+    for (int i = 0; i < 3 && g1.small_boxes; ++i) {
+      rc = make_map_u8(&g1.map_x_lo_small[i], xq_lo, l.capacity, c.hidden, 16 << i);
+      if (rc) return rc;
+    }
     g1.x_scale_lo = xs_lo;
     g1.out_q_lo = hq_lo;
     g1.out_scale_lo = hs_lo;
@@ -626,15 +630,19 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
   if (rc) return rc;
   rc = make_map_u8(&g2.map_x, ws + l.hq, l.capacity, c.inter, 128);
   if (rc) return rc;
-  rc = make_map_u8(&g2.map_x_rows32, ws + l.hq, l.capacity, c.inter, 32);
-  if (rc) return rc;
-  rc = make_map_u8(&g2.map_x_rows64, ws + l.hq, l.capacity, c.inter, 64);
-  if (rc) return rc;
-  g2.small_boxes = small_activation_boxes(c) && !split;
+  g2.small_boxes = small_activation_boxes(c);
+  for (int i = 0; i < 3 && g2.small_boxes; ++i) {
+    rc = make_map_u8(&g2.map_x_small[i], ws + l.hq, l.capacity, c.inter, 16 << i);
+    if (rc) return rc;
+  }
   g2.split = split;
   if (split) {
     rc = make_map_u8(&g2.map_x_lo, hq_lo, l.capacity, c.inter, 128);
     if (rc) return rc;
+    for (int i = 0; i < 3 && g2.small_boxes; ++i) {
+      rc = make_map_u8(&g2.map_x_lo_small[i], hq_lo, l.capacity, c.inter, 16 << i);
+      if (rc) return rc;
+    }
     g2.x_scale_lo = hs_lo;
   }
   g2.w_scale = w2_scale;

@@ -106,13 +106,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Whether the producer loads row `row` of the sorted table when blocks with at most 32 / 64 routed rows load only
-// those (a block's routed rows come first).
+// Which box the producer loads of the 128-row block that starts at row `b0` of the sorted table, when blocks with few
+// routed rows load only those (a block's routed rows come first): 0, 1, 2 = 16, 32, 64 rows, 3 = all 128.
+__device__ __forceinline__ int small_box_index(const int32_t* sorted_ids, int b0) {
+  const int id16 = sorted_ids[b0 + 16], id32 = sorted_ids[b0 + 32], id64 = sorted_ids[b0 + 64];
+  return id16 < 0 ? 0 : id32 < 0 ? 1 : id64 < 0 ? 2 : 3;
+}
+// Whether the producer then loads row `row`.
 __device__ __forceinline__ bool row_in_small_box(const int32_t* sorted_ids, int row) {
-  const int r = row & 127, b0 = row & ~127;
-  if (r < 32) return true;
-  if (sorted_ids[b0 + 32] < 0) return false;
-  return r < 64 || sorted_ids[b0 + 64] >= 0;
+  return (row & 127) < (16 << small_box_index(sorted_ids, row & ~127));
 }
 
 // ue8m0 exponent of the smallest power of two >= amax / 448 (frexp rule of the reference's _mxfp8):
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
   }
-  // A block with few routed rows loads a 32- or 64-row box; the MMA still multiplies all 128 rows of the stage.
+  // A block with few routed rows loads a 16-, 32- or 64-row box; the MMA still multiplies all 128 rows of the stage.
   // Start them as zeros: in a decode batch, where every block is such a block, they stay zero, and what the tensor
   // core draws -- and with it the clock the part holds -- depends on the operands.
   for (int s = 0; s < S; ++s)
@@ -241,14 +243,17 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
       // A decode batch leaves most of a 128-row block as padding (the sort puts the routed rows
       // first, -1 after them).  Loading all 128 activation rows per K-block made shared-memory
       // fill traffic from L2, not HBM, the bound (32 KB per K-block against 16 KB of weights): a
-      // block with at most 32 or 64 routed rows loads only those.  The rows left stale feed TMEM
+      // block with at most 16, 32 or 64 routed rows loads only those.  The rows left stale feed TMEM
       // lanes whose results are never stored.
-      const CUtensorMap* map_x = &p.map_x;
+      const CUtensorMap *map_x = &p.map_x, *map_x_lo = &p.map_x_lo;
       uint32_t x_bytes = kABytes;
-      if (!SPLIT && p.small_boxes) {
-        const int id32 = p.sorted_ids[b * kBM + 32], id64 = p.sorted_ids[b * kBM + 64];
-        if (id32 < 0) { map_x = &p.map_x_rows32; x_bytes = 32 * 128; }
-        else if (id64 < 0) { map_x = &p.map_x_rows64; x_bytes = 64 * 128; }
+      if (p.small_boxes) {
+        const int box = small_box_index(p.sorted_ids, b * kBM);
+        if (box < 3) {
+          map_x = &p.map_x_small[box];
+          map_x_lo = &p.map_x_lo_small[box];
+          x_bytes = (16 << box) * 128;
+        }
       }
       for (int kb = 0; kb < KB; ++kb) {
         if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, p.status, 21)) { ok = false; break; }
@@ -258,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
           // global memory), not the padded bytes it writes: expecting the padded size never completes
           mbar_expect_tx(&full[s], (SPLIT ? 2 : 1) * x_bytes + kBBytes / 2);
           tma_load_2d(st, map_x, &full[s], kb * 128, b * kBM);
-          if (SPLIT) tma_load_2d(st + kABytes, &p.map_x_lo, &full[s], kb * 128, b * kBM);
+          if (SPLIT) tma_load_2d(st + kABytes, map_x_lo, &full[s], kb * 128, b * kBM);
           if (GATE_UP) {
             tma_load_2d(st + kOffB, &p.map_w, &full[s], kb * 128, w_row);
             tma_load_2d(st + kOffB + kBBytes / 2, &p.map_w, &full[s], kb * 128, w_row + p.out_dim);
@@ -396,11 +401,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
         wgt_s[et] = rid < 0 ? 0.0f : (weights ? weights[rid] : 1.0f);
       }
       // gate_up: rows the down projection's producer will load (padding rows among them get zero codes)
-      int box_rows = kBM;
-      if (GATE_UP && !SPLIT && p.small_boxes) {
-        if (p.sorted_ids[b * kBM + 32] < 0) box_rows = 32;
-        else if (p.sorted_ids[b * kBM + 64] < 0) box_rows = 64;
-      }
+      const int box_rows = GATE_UP && p.small_boxes ? 16 << small_box_index(p.sorted_ids, b * kBM) : kBM;
       epi_sync();  // the epilogue reads other threads' entries
       // ---- epilogue: the whole K reduction is in TMEM ----
       {
@@ -558,88 +559,92 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
   }
 }
 
-// Four lanes x 8 values per 1 x 32 group: rows
-// gathered through the sorted route table, e4m3 codes row-major, scale bytes in tcgen05.cp order.
+// Four lanes x 8 values per 1 x 32 group: rows gathered through the sorted route table, e4m3 codes row-major, scale
+// bytes in tcgen05.cp order.  A CTA column works on one 128-row block: its routed rows come first, so their count -- one
+// look at the block's ids -- is all the work there is, plus zero codes for the padding rows that the GEMM's producer
+// loads.  A warp takes 1024 values of a row at a time, all four 16-byte loads of a lane in flight.  (Walking every row
+// of the table, padding included, took 65 us for 64 tokens on 231 experts, of which 576 rows of 29.6 k are routed.)
+constexpr int kMxQuantSegment = 1024;  // values of a row per warp and pass
 __global__ void __launch_bounds__(256) gather_quant_mxfp8_kernel(MxQuantParams p) {
   griddep_wait();
   griddep_launch();
   const int groups_per_row = p.hidden >> 5;
-  const int n_rows = p.num_rows ? min(*p.num_rows, p.n_rows) : p.n_rows;
-  const int64_t total = static_cast<int64_t>(n_rows) * groups_per_row;
-  const int sub = threadIdx.x & 3;
-  const uint32_t group_mask = 0xFu << (threadIdx.x & 28);
-  const int64_t quads = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 2;
   const int KB = p.hidden >> 7;
-  for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 2; g < total; g += quads) {
-    const int row = static_cast<int>(static_cast<uint32_t>(g) / static_cast<uint32_t>(groups_per_row));  // total < 2^31: checked at launch
-    const int grp = static_cast<int>(static_cast<uint32_t>(g) - static_cast<uint32_t>(row) * static_cast<uint32_t>(groups_per_row));
-    const int rid = p.sorted_ids ? p.sorted_ids[row] : row;  // no table: quantise the rows in place order
-    if (rid < 0) {
-      if (p.zero_padding == 1 || (p.zero_padding == 2 && row_in_small_box(p.sorted_ids, row))) {
-        *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(row) * p.hidden + grp * 32 + sub * 8) = make_uint2(0u, 0u);
-        if (p.q_lo) *reinterpret_cast<uint2*>(p.q_lo + static_cast<size_t>(row) * p.hidden + grp * 32 + sub * 8) = make_uint2(0u, 0u);
-      }
-      continue;
-    }
-    const int token = rid / p.routes_per_token;
-    if (p.q_in) {  // rows quantised by their sender: move codes and scale byte
-      *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(row) * p.hidden + grp * 32 + sub * 8) =
-          *reinterpret_cast<const uint2*>(p.q_in + static_cast<size_t>(token) * p.hidden + grp * 32 + sub * 8);
-      if (sub == 0) {
-        const int b = row >> 7, r = row & 127, kb = grp >> 2, ks = grp & 3;
-        p.scales[(static_cast<size_t>(b) * KB + kb) * kSfaBytes + (r & 31) * 16 + (r >> 5) * 4 + ks] =
-            p.scales_in[static_cast<size_t>(token) * groups_per_row + grp];
-      }
-      continue;
-    }
-    const uint4 raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x) +
-                                                      static_cast<size_t>(token) * p.hidden + grp * 32 + sub * 8);
-    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-    float v[8];
-    float m = 0.0f;
+  const int n_rows = p.num_rows ? min(*p.num_rows, p.n_rows) : p.n_rows;
+  const int lane = threadIdx.x & 31, sub = threadIdx.x & 3;
+  const uint32_t group_mask = 0xFu << (threadIdx.x & 28);
+  const int segments = (p.hidden + kMxQuantSegment - 1) / kMxQuantSegment;
+  const int first_item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), item_step = gridDim.y * (blockDim.x >> 5);
+  for (int row0 = blockIdx.x * 128; row0 < n_rows; row0 += gridDim.x * 128) {
+    int live = min(128, n_rows - row0);
+    if (p.num_rows)  // a table the sort made; one that a caller made may hold its -1 rows anywhere
+      live = __syncthreads_count(threadIdx.x < live && p.sorted_ids[row0 + threadIdx.x] >= 0);
+    for (int item = first_item; item < live * segments; item += item_step) {
+      const int row = row0 + item / segments;
+      const int c0 = item % segments * kMxQuantSegment + lane * 8;  // this lane's first value; the others 256 apart
+      const int rid = p.sorted_ids ? p.sorted_ids[row] : row;  // no table: quantise the rows in place order
+      if (rid < 0) continue;
+      const int token = rid / p.routes_per_token;
+      const uint16_t* x = reinterpret_cast<const uint16_t*>(p.x) + static_cast<size_t>(token) * p.hidden;
+      uint4 raw[kMxQuantSegment / 256];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      v[2 * i] = __uint_as_float(w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-      m = fmaxf(m, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-    }
-    m = fmaxf(m, __shfl_xor_sync(group_mask, m, 2, 4));
-    m = fmaxf(m, __shfl_xor_sync(group_mask, m, 1, 4));
-    const int ex = p.act_fp4 ? mxfp4_exponent(m) : mxfp8_exponent(m);
-    const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
-    uint2 out;
-    if (p.act_fp4) {
-      out.x = e2m1_grid_as_e4m3x2(v[0] * inv, v[1] * inv) | (static_cast<uint32_t>(e2m1_grid_as_e4m3x2(v[2] * inv, v[3] * inv)) << 16);
-      out.y = e2m1_grid_as_e4m3x2(v[4] * inv, v[5] * inv) | (static_cast<uint32_t>(e2m1_grid_as_e4m3x2(v[6] * inv, v[7] * inv)) << 16);
-    } else if (p.q_lo) {  // the value itself, as two e4m3 terms
-      const int ex_lo = ex - 4 < -127 ? -127 : ex - 4;
-      const float lo_mul = __uint_as_float(static_cast<uint32_t>(127 + ex - ex_lo) << 23);
-      uint16_t hi[4], lo[4];
+      for (int u = 0; u < kMxQuantSegment / 256; ++u)
+        if (c0 + u * 256 < p.hidden) raw[u] = *reinterpret_cast<const uint4*>(x + c0 + u * 256);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) e4m3x2_two_terms(v[2 * i] * inv, v[2 * i + 1] * inv, lo_mul, hi[i], lo[i]);
-      out.x = hi[0] | (static_cast<uint32_t>(hi[1]) << 16);
-      out.y = hi[2] | (static_cast<uint32_t>(hi[3]) << 16);
-      uint2 out_lo;
-      out_lo.x = lo[0] | (static_cast<uint32_t>(lo[1]) << 16);
-      out_lo.y = lo[2] | (static_cast<uint32_t>(lo[3]) << 16);
-      *reinterpret_cast<uint2*>(p.q_lo + static_cast<size_t>(row) * p.hidden + grp * 32 + sub * 8) = out_lo;
-      if (sub == 0) {
+      for (int u = 0; u < kMxQuantSegment / 256; ++u) {
+        const int col = c0 + u * 256, grp = col >> 5;
+        if (col >= p.hidden) continue;  // uniform over a group's four lanes: hidden is a multiple of 128
+        const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+        float v[8];
+        float m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          v[2 * i] = __uint_as_float(w[i] << 16);
+          v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+          m = fmaxf(m, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
+        }
+        m = fmaxf(m, __shfl_xor_sync(group_mask, m, 2, 4));
+        m = fmaxf(m, __shfl_xor_sync(group_mask, m, 1, 4));
+        const int ex = p.act_fp4 ? mxfp4_exponent(m) : mxfp8_exponent(m);
+        const float inv = __uint_as_float(static_cast<uint32_t>(127 - ex) << 23);
+        const size_t at = static_cast<size_t>(row) * p.hidden + col;
         const int b = row >> 7, r = row & 127, kb = grp >> 2, ks = grp & 3;
-        p.scales_lo[(static_cast<size_t>(b) * KB + kb) * kSfaBytes + (r & 31) * 16 + (r >> 5) * 4 + ks] =
-            static_cast<uint8_t>(ex_lo + 127);
+        const size_t scale_at = p.row_major_scales  // for transport to another rank: [row, hidden/32]
+                                    ? static_cast<size_t>(row) * groups_per_row + grp
+                                    : (static_cast<size_t>(b) * KB + kb) * kSfaBytes + (r & 31) * 16 + (r >> 5) * 4 + ks;
+        uint2 out;
+        if (p.act_fp4) {
+          out.x = e2m1_grid_as_e4m3x2(v[0] * inv, v[1] * inv) | (static_cast<uint32_t>(e2m1_grid_as_e4m3x2(v[2] * inv, v[3] * inv)) << 16);
+          out.y = e2m1_grid_as_e4m3x2(v[4] * inv, v[5] * inv) | (static_cast<uint32_t>(e2m1_grid_as_e4m3x2(v[6] * inv, v[7] * inv)) << 16);
+        } else if (p.q_lo) {  // the value itself, as two e4m3 terms
+          const int ex_lo = ex - 4 < -127 ? -127 : ex - 4;
+          const float lo_mul = __uint_as_float(static_cast<uint32_t>(127 + ex - ex_lo) << 23);
+          uint16_t hi[4], lo[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) e4m3x2_two_terms(v[2 * i] * inv, v[2 * i + 1] * inv, lo_mul, hi[i], lo[i]);
+          out.x = hi[0] | (static_cast<uint32_t>(hi[1]) << 16);
+          out.y = hi[2] | (static_cast<uint32_t>(hi[3]) << 16);
+          uint2 out_lo;
+          out_lo.x = lo[0] | (static_cast<uint32_t>(lo[1]) << 16);
+          out_lo.y = lo[2] | (static_cast<uint32_t>(lo[3]) << 16);
+          *reinterpret_cast<uint2*>(p.q_lo + at) = out_lo;
+          if (sub == 0) p.scales_lo[scale_at] = static_cast<uint8_t>(ex_lo + 127);
+        } else {
+          out.x = cvt_e4m3x2(v[0] * inv, v[1] * inv) | (static_cast<uint32_t>(cvt_e4m3x2(v[2] * inv, v[3] * inv)) << 16);
+          out.y = cvt_e4m3x2(v[4] * inv, v[5] * inv) | (static_cast<uint32_t>(cvt_e4m3x2(v[6] * inv, v[7] * inv)) << 16);
+        }
+        *reinterpret_cast<uint2*>(p.q + at) = out;
+        if (sub == 0) p.scales[scale_at] = static_cast<uint8_t>(ex + 127);
       }
-    } else {
-      out.x = cvt_e4m3x2(v[0] * inv, v[1] * inv) | (static_cast<uint32_t>(cvt_e4m3x2(v[2] * inv, v[3] * inv)) << 16);
-      out.y = cvt_e4m3x2(v[4] * inv, v[5] * inv) | (static_cast<uint32_t>(cvt_e4m3x2(v[6] * inv, v[7] * inv)) << 16);
     }
-    *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(row) * p.hidden + grp * 32 + sub * 8) = out;
-    if (sub == 0) {
-      if (p.row_major_scales) {  // for transport to another rank: [row, hidden/32]
-        p.scales[static_cast<size_t>(row) * groups_per_row + grp] = static_cast<uint8_t>(ex + 127);
-      } else {
-        const int b = row >> 7, r = row & 127, kb = grp >> 2, ks = grp & 3;
-        p.scales[(static_cast<size_t>(b) * KB + kb) * kSfaBytes + (r & 31) * 16 + (r >> 5) * 4 + ks] =
-            static_cast<uint8_t>(ex + 127);
+    if (p.num_rows && p.zero_padding) {
+      const int loaded = p.zero_padding == 1 ? 128 : 16 << small_box_index(p.sorted_ids, row0);
+      const int vec_per_row = p.hidden >> 4;
+      uint4* z = reinterpret_cast<uint4*>(p.q + static_cast<size_t>(row0) * p.hidden);
+      uint4* z_lo = p.q_lo ? reinterpret_cast<uint4*>(p.q_lo + static_cast<size_t>(row0) * p.hidden) : nullptr;
+      for (int i = live * vec_per_row + blockIdx.y * blockDim.x + threadIdx.x; i < loaded * vec_per_row; i += gridDim.y * blockDim.x) {
+        z[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (z_lo) z_lo[i] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
   }
@@ -716,11 +721,13 @@ int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream) {
     const int grid = static_cast<int>(blocks < 148 * 32 ? blocks : 148 * 32);
     return launch_kernel(gather_rows_mxfp8_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
   }
-  const int64_t groups = static_cast<int64_t>(p.n_rows) * (p.hidden / 32);
-  if (groups >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
-  const int64_t blocks = (groups * 4 + 255) / 256;
-  const int grid = static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16);
-  return launch_kernel(gather_quant_mxfp8_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  if (static_cast<int64_t>(p.n_rows) * (p.hidden / 32) >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
+  // one CTA column per 128-row block; where the blocks are few, several CTAs share a block's rows
+  const int64_t blocks = (static_cast<int64_t>(p.n_rows) + 127) / 128;
+  const int grid = static_cast<int>(blocks < 65535 ? blocks : 65535);
+  int share = 148 * 8 / grid;
+  share = share < 1 ? 1 : share > 32 ? 32 : share;
+  return launch_kernel(gather_quant_mxfp8_kernel, dim3(grid, share), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 int grouped_gemm_mx_pick_stages(bool gate_up, bool split) {

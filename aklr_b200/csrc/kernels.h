@@ -149,7 +149,7 @@ struct MxQuantParams {
   int act_fp4;
   // Padding rows of the table that the GEMM's producer loads get zero codes (they are multiplied although never
   // read back, and zero operands cost the tensor core least): 0 off, 1 every padding row, 2 only those inside the
-  // 32- or 64-row box of a block with that few routed rows (MxGemmParams::small_boxes).
+  // 16-, 32- or 64-row box of a block with that few routed rows (MxGemmParams::small_boxes).
   int zero_padding;
 };
 int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream);
@@ -157,9 +157,9 @@ int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream);
 struct MxGemmParams {
   CUtensorMap map_w;           // packed e2m1 weights [experts*rows_per_expert, k], 16U4_ALIGN16B, box 128 x 128|256
   CUtensorMap map_x;           // e4m3 activations [capacity, k], box 128 x 128
-  CUtensorMap map_x_rows32;    // the same matrix with boxes of 32 and 64 rows: a block with that few routed
-  CUtensorMap map_x_rows64;    // rows loads only those (the tile's other rows are never read back)
-  int small_boxes;             // non-zero: the two maps above are set
+  CUtensorMap map_x_small[3];  // the same matrix with boxes of 16, 32 and 64 rows: a block with that few routed
+                               // rows loads only those (the tile's other rows are never read back)
+  int small_boxes;             // non-zero: the three maps above are set (and, with split, map_x_lo_small)
   const uint8_t* w_scale;      // e8m0 [experts, rows_per_expert, k/32]
   const uint8_t* x_scale;      // e8m0 [max_blocks, k/128, 512]
   const int32_t* sorted_ids;
@@ -180,7 +180,7 @@ struct MxGemmParams {
   // for gate_up, outputs; split != 0 issues two MMAs per K step on the same weight tile
   int split;
   int act_fp4;  // gate_up: requantise the gated product to the MXFP4 grid (see MxQuantParams)
-  CUtensorMap map_x_lo;
+  CUtensorMap map_x_lo, map_x_lo_small[3];
   const uint8_t* x_scale_lo;
   uint8_t* out_q_lo;
   uint8_t* out_scale_lo;
