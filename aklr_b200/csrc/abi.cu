@@ -127,6 +127,21 @@ int make_map_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t co
   return AKLR_OK;
 }
 
+// float32 matrix [rows, cols]: box = box_rows x 64 elements, rows one after the other, zero fill outside.
+int make_map_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeTiledFn encode = encode_tiled_fn();
+  if (!encode) return fail(AKLR_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {cols * 4};
+  const cuuint32_t box[2] = {64, box_rows};
+  const cuuint32_t elem[2] = {1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(AKLR_ERR_CUDA, "cuTensorMapEncodeTiled (float32) failed with CUresult %d", (int)r);
+  return AKLR_OK;
+}
+
 int sm_count() {
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -1270,7 +1285,19 @@ int aklr_router_gemm_f32(const void* x, const float* w, float* logits, int32_t n
   if (!x || !w || !logits) return fail(AKLR_ERR_BAD_ARGUMENT, "NULL argument");
   int rc = check_device();
   if (rc) return rc;
-  rc = aklr::launch_router_gemm_f32(x, w, logits, n_tokens, hidden, n_routed, static_cast<cudaStream_t>(stream));
+  // From 17 tokens on the tensor cores; below them, and for token rows that a TMA load cannot start at, dot products.
+  if (n_tokens > 16 && n_routed >= 1 && hidden % 128 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
+      reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0) {
+    CUtensorMap map_x, map_w;
+    rc = make_map_bf16(&map_x, x, n_tokens, hidden, 128);
+    if (rc) return rc;
+    rc = make_map_f32(&map_w, w, n_routed, hidden, 32);
+    if (rc) return rc;
+    rc = aklr::launch_router_gemm_f32_tc(map_x, map_w, logits, n_tokens, hidden, n_routed,
+                                         aklr::host_visible_status(static_cast<cudaStream_t>(stream)), static_cast<cudaStream_t>(stream));
+  } else {
+    rc = aklr::launch_router_gemm_f32(x, w, logits, n_tokens, hidden, n_routed, static_cast<cudaStream_t>(stream));
+  }
   if (rc) return fail(rc, "router GEMM (float32 weights): %s", aklr_status_string(rc));
   g_launches += n_tokens > 0;
   return AKLR_OK;

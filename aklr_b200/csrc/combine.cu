@@ -275,7 +275,8 @@ int launch_add_gated_rows(const void* x, const void* gate, const void* rows, voi
 // aklr/plugins/sglang/models/minimax_m2/reference.py:43-50 takes x @ router^T in float32, nothing
 // rounded).  CUDA cores, float32 FMAs in k order.
 //  * few tokens: one warp per (token, expert) dot product, so the weight is read by many SMs;
-//  * else a 64 x 64 tile per CTA, 16 k per step through shared memory, 4 x 4 outputs per thread.
+//  * else the tensor cores (router_gemm.cu); this file keeps a 64 x 64 tile per CTA, 16 k per step, 4 x 4 outputs per
+//    thread, for token rows a TMA load cannot start at.
 __global__ void __launch_bounds__(256)
 router_dot_f32_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,
                       int n_tokens, int hidden, int n_routed) {
