@@ -236,9 +236,16 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
     int s = 0;  // ring position and the parity of its current use
     uint32_t ph = 0;
     bool ok = true;
+    // A tile's expert and box are read during the tile before it: a short reduction (2 K-blocks at an intermediate
+    // width of 256) is over before such a load returns.
+    auto expert_of = [&](int t) { return t < total_tiles ? p.block_expert[t / tiles_per_block] : 0; };
+    auto box_of = [&](int t) { return p.small_boxes && t < total_tiles ? small_box_index(p.sorted_ids, t / tiles_per_block * kBM) : 3; };
+    int e_next = expert_of(blockIdx.x), box_next = box_of(blockIdx.x);
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       const int b = t / tiles_per_block, j = t - b * tiles_per_block;
-      const int e = p.block_expert[b];
+      const int e = e_next, box = box_next;
+      e_next = expert_of(t + gridDim.x);
+      box_next = box_of(t + gridDim.x);
       const int w_row = e * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256);
       // A decode batch leaves most of a 128-row block as padding (the sort puts the routed rows
       // first, -1 after them).  Loading all 128 activation rows per K-block made shared-memory
@@ -247,13 +254,10 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
       // lanes whose results are never stored.
       const CUtensorMap *map_x = &p.map_x, *map_x_lo = &p.map_x_lo;
       uint32_t x_bytes = kABytes;
-      if (p.small_boxes) {
-        const int box = small_box_index(p.sorted_ids, b * kBM);
-        if (box < 3) {
-          map_x = &p.map_x_small[box];
-          map_x_lo = &p.map_x_lo_small[box];
-          x_bytes = (16 << box) * 128;
-        }
+      if (box < 3) {
+        map_x = &p.map_x_small[box];
+        map_x_lo = &p.map_x_lo_small[box];
+        x_bytes = (16 << box) * 128;
       }
       for (int kb = 0; kb < KB; ++kb) {
         if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, p.status, 21)) { ok = false; break; }
@@ -319,64 +323,73 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
     // ------------------- scale-factor staging, running ahead of the MMA warp -------------------
     // The two staging warps take alternate K-blocks, so each has two MMA periods per stage; a
     // lane moves 8 weight-row words (rows lane, lane+32, ...) and 16 bytes of activation scales.
+    // Their K-blocks are one stream across the CTA's tiles: a warp's loads run kDepth of its own K-blocks ahead of its
+    // stores whatever tile those belong to, and a tile's expert is read a tile before its addresses are formed.  (With the
+    // ring refilled per tile every tile began with two dependent memory round trips, 2000-2500 cycles: at 2 K-blocks a
+    // tile that was most of its time.)
     const int sw = warp - 10;
     const int KS = p.k >> 5;  // scale bytes per weight row
-    uint32_t it0 = 0;         // K-blocks before this tile
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, it0 += KB) {
-      const int b = t / tiles_per_block, j = t - b * tiles_per_block;
-      const int e = p.block_expert[b];
-      const uint8_t* wsf[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int i = lane + q * 32;
-        const int wrow = GATE_UP ? (i < 128 ? j * 128 + i : p.out_dim + j * 128 + (i - 128)) : j * 256 + i;
-        wsf[q] = p.w_scale + (static_cast<size_t>(e) * p.rows_per_expert + wrow) * KS;
+    // rows lane, lane + 32, ... of the tile's 256; gate_up: the up rows start out_dim rows after the gate rows
+    const size_t row_step = static_cast<size_t>(32) * KS;
+    const size_t second_half = GATE_UP ? static_cast<size_t>(p.out_dim - 128) * KS : 0;
+    int ld_t = blockIdx.x, ld_kb = sw;  // where the next load is
+    int e_ahead = ld_t < total_tiles ? p.block_expert[ld_t / tiles_per_block] : 0;
+    const uint8_t *wsf = nullptr, *xsf = nullptr, *xsf_lo = nullptr;
+    auto point = [&] {  // addresses of tile ld_t, whose expert is e_ahead
+      if (ld_t >= total_tiles) return;
+      const int b = ld_t / tiles_per_block, j = ld_t - b * tiles_per_block;
+      wsf = p.w_scale + (static_cast<size_t>(e_ahead) * p.rows_per_expert + (GATE_UP ? j * 128 : j * 256) + lane) * KS;
+      xsf = p.x_scale + static_cast<size_t>(b) * KB * kSfaBytes + lane * 16;
+      if (SPLIT) xsf_lo = p.x_scale_lo + static_cast<size_t>(b) * KB * kSfaBytes + lane * 16;
+      const int next = ld_t + gridDim.x;
+      e_ahead = next < total_tiles ? p.block_expert[next / tiles_per_block] : 0;
+    };
+    auto carry = [&] {  // ld_kb past the tile's end: on to the tile it falls in
+      while (ld_kb >= KB && ld_t < total_tiles) {
+        ld_kb -= KB;
+        ld_t += gridDim.x;
+        point();
       }
-      const uint8_t* xsf = p.x_scale + static_cast<size_t>(b) * KB * kSfaBytes;
-      const uint8_t* xsf_lo = SPLIT ? p.x_scale_lo + static_cast<size_t>(b) * KB * kSfaBytes : nullptr;
-      const int first = ((it0 & 1u) == static_cast<uint32_t>(sw)) ? 0 : 1;
-      // ring of kDepth own K-blocks of scale words in registers: loaded long before their stage
-      // frees up (down-projection rows are 64 bytes apart and miss to HBM on first touch)
-      constexpr int kDepth = 3;
-      uint32_t wq[kDepth][8];
-      uint4 aq[kDepth], aq_lo[SPLIT ? kDepth : 1];
+    };
+    constexpr int kDepth = 3;
+    uint32_t wq[kDepth][8];
+    uint4 aq[kDepth], aq_lo[SPLIT ? kDepth : 1];
+    auto load = [&](uint32_t (&w)[8], uint4& a, uint4& a_lo) {
+      if (ld_t >= total_tiles) return;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        w[q] = __ldg(reinterpret_cast<const uint32_t*>(wsf + q * row_step + (q >= 4 ? second_half : 0) + ld_kb * 4));
+      a = __ldg(reinterpret_cast<const uint4*>(xsf + ld_kb * kSfaBytes));
+      if (SPLIT) a_lo = __ldg(reinterpret_cast<const uint4*>(xsf_lo + ld_kb * kSfaBytes));
+      ld_kb += 2;
+      carry();
+    };
+    point();
+    carry();
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) load(wq[d], aq[d], aq_lo[SPLIT ? d : 0]);
+    const int my_tiles = static_cast<int>(blockIdx.x) < total_tiles ? (total_tiles - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1 : 0;
+    const int total_its = my_tiles * KB;  // K-blocks of this CTA
+    int s = sw % S;                       // ring position and parity of K-block `it`
+    uint32_t ph = (sw / S) & 1;
+    bool ok = true;
+    for (int it0 = sw; it0 < total_its && ok; it0 += 2 * kDepth) {
 #pragma unroll
       for (int d = 0; d < kDepth; ++d) {
-        const int kb = first + 2 * d;
+        if (it0 + 2 * d < total_its && ok) {
+          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 25)) ok = false;
+          uint8_t* sf = smem + s * kStageBytes + kOffSf;
+          *reinterpret_cast<uint4*>(sf + lane * 16) = aq[d];
+          if (SPLIT) *reinterpret_cast<uint4*>(sf + kSfLoOffset + lane * 16) = aq_lo[SPLIT ? d : 0];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) wq[d][q] = kb < KB ? __ldg(reinterpret_cast<const uint32_t*>(wsf[q] + kb * 4)) : 0u;
-        aq[d] = kb < KB ? __ldg(reinterpret_cast<const uint4*>(xsf + kb * kSfaBytes) + lane) : make_uint4(0, 0, 0, 0);
-        if (SPLIT) aq_lo[d] = kb < KB ? __ldg(reinterpret_cast<const uint4*>(xsf_lo + kb * kSfaBytes) + lane) : make_uint4(0, 0, 0, 0);
-      }
-      for (int kb0 = first; kb0 < KB && ok; kb0 += 2 * kDepth) {
-#pragma unroll
-        for (int d = 0; d < kDepth; ++d) {
-          const int kb = kb0 + 2 * d;
-          if (kb < KB && ok) {
-            const uint32_t it = it0 + kb;
-            const int s = it % S;
-            const uint32_t ph = (it / S) & 1;
-            bool got;
-            got = mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 25);
-            if (!got) ok = false;
-            uint8_t* sf = smem + s * kStageBytes + kOffSf;
-            *reinterpret_cast<uint4*>(sf + lane * 16) = aq[d];
-            if (SPLIT) *reinterpret_cast<uint4*>(sf + kSfLoOffset + lane * 16) = aq_lo[d];
-#pragma unroll
-            for (int q = 0; q < 8; ++q)  // row lane + 32 q -> 16-byte line `lane`, word q % 4, chunk q / 4
-              *reinterpret_cast<uint32_t*>(sf + kSfaBytes + (q >> 2) * 512 + lane * 16 + (q & 3) * 4) = wq[d][q];
-            fence_proxy_async_smem();  // tcgen05.cp reads these bytes through the async proxy
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sf_full[s]);
-            const int nk = kb + 2 * kDepth;
-            if (nk < KB) {
-#pragma unroll
-              for (int q = 0; q < 8; ++q) wq[d][q] = __ldg(reinterpret_cast<const uint32_t*>(wsf[q] + nk * 4));
-              aq[d] = __ldg(reinterpret_cast<const uint4*>(xsf + nk * kSfaBytes) + lane);
-              if (SPLIT) aq_lo[d] = __ldg(reinterpret_cast<const uint4*>(xsf_lo + nk * kSfaBytes) + lane);
-            }
-          }
+          for (int q = 0; q < 8; ++q)  // row lane + 32 q -> 16-byte line `lane`, word q % 4, chunk q / 4
+            *reinterpret_cast<uint32_t*>(sf + kSfaBytes + (q >> 2) * 512 + lane * 16 + (q & 3) * 4) = wq[d][q];
+          fence_proxy_async_smem();  // tcgen05.cp reads these bytes through the async proxy
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sf_full[s]);
+          s += 2;
+          if (s >= S) { s -= S; ph ^= 1; }
+          load(wq[d], aq[d], aq_lo[SPLIT ? d : 0]);
         }
       }
     }
@@ -389,27 +402,53 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
     uint32_t tile_no = 0;
     bool bad = false;
+    // down: the route weight, or 1 when the gate_up projection already carried it; gate_up: the
+    // route weight when it is applied there (doweight_stage1), else 1
+    const float* weights = GATE_UP ? p.stage1_weights : p.topk_weights;
+    // A tile's route ids, route weights and box are loaded during the tile before it.
+    auto rid_of = [&](int t) { return t < total_tiles && et < kBM ? p.sorted_ids[t / tiles_per_block * kBM + et] : -1; };
+    auto weight_of = [&](int rid) { return rid < 0 ? 0.0f : (weights ? weights[rid] : 1.0f); };
+    // gate_up: rows the down projection's producer will load (padding rows among them get zero codes)
+    auto box_of = [&](int t) {
+      return GATE_UP && p.small_boxes && t < total_tiles ? 16 << small_box_index(p.sorted_ids, t / tiles_per_block * kBM) : kBM;
+    };
+    int rid_next = rid_of(blockIdx.x), box_next = box_of(blockIdx.x);
+    float weight_next = weight_of(rid_next);
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_no) {
       if (epi_any(*abort_flag)) break;
       const int b = t / tiles_per_block, j = t - b * tiles_per_block;
       if (et < kBM) {
-        const int rid = p.sorted_ids[b * kBM + et];
-        rid_s[et] = rid;
-        // down: the route weight, or 1 when the gate_up projection already carried it; gate_up: the
-        // route weight when it is applied there (doweight_stage1), else 1
-        const float* weights = GATE_UP ? p.stage1_weights : p.topk_weights;
-        wgt_s[et] = rid < 0 ? 0.0f : (weights ? weights[rid] : 1.0f);
+        rid_s[et] = rid_next;
+        wgt_s[et] = weight_next;
       }
-      // gate_up: rows the down projection's producer will load (padding rows among them get zero codes)
-      const int box_rows = GATE_UP && p.small_boxes ? 16 << small_box_index(p.sorted_ids, b * kBM) : kBM;
+      const int box_rows = box_next;
+      rid_next = rid_of(t + gridDim.x);
+      box_next = box_of(t + gridDim.x);
       epi_sync();  // the epilogue reads other threads' entries
+      const int rid = rid_s[row];
+      const bool warp_has_rows = __any_sync(0xFFFFFFFFu, rid >= 0);
       // ---- epilogue: the whole K reduction is in TMEM ----
       {
         bool got;
         got = mbar_wait(acc_full, tile_no & 1, abort_flag, p.status, 26);
         if (!got) bad = true;
       }
+      weight_next = weight_of(rid_next);
       tc_fence_after_sync();
+      if (!warp_has_rows) {  // a block's routed rows come first: this warp's 32 rows are all padding and nothing reads their results
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
+        if (GATE_UP && row < box_rows && !bad) {
+          const size_t at = static_cast<size_t>(b * kBM + row) * p.out_dim + j * 128 + half * 64;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            *reinterpret_cast<uint4*>(p.out_q + at + v * 16) = make_uint4(0u, 0u, 0u, 0u);
+            if (SPLIT) *reinterpret_cast<uint4*>(p.out_q_lo + at + v * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+        }
+        continue;
+      }
       float acc[128];
       {
         // tcgen05.ld is latency-bound: all eight loads in flight, one wait, so that the accumulator
@@ -429,7 +468,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty);
 
-      const int rid = rid_s[row];
       if (GATE_UP) {
         const int IB = p.out_dim >> 7;
         const float w1row = p.stage1_weights ? wgt_s[row] : 1.0f;  // exact when the weight is not applied here
