@@ -567,9 +567,11 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
     qp.q_lo = xq_lo;
     qp.scales_lo = xs_lo;
   }
-  if (!split && !q_in && routes_per_token > 1 && c.n_tokens >= kQuantOncePerTokenFrom) {
+  if (!q_in && routes_per_token > 1 && c.n_tokens >= kQuantOncePerTokenFrom) {
     // quantise every token once (codes and row-major scale bytes parked in the space of the
-    // per-route output rows, unused until the down projection), then copy per route
+    // per-route output rows, unused until the down projection), then copy per route; with activations
+    // kept in bf16 the two terms' planes are copied one after the other (1001 tokens x 8 routes on 6144: 100 us when
+    // every route split its token again)
     uint8_t* tq = ws + l.rows;
     uint8_t* ts = tq + align_up(static_cast<int64_t>(c.n_tokens) * c.hidden, 256);
     MxQuantParams tp{};
@@ -581,9 +583,26 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
     tp.routes_per_token = 1;
     tp.row_major_scales = 1;
     tp.act_fp4 = fp4;
+    uint8_t* tq_lo = ts + align_up(static_cast<int64_t>(c.n_tokens) * (c.hidden / 32), 256);
+    uint8_t* ts_lo = tq_lo + align_up(static_cast<int64_t>(c.n_tokens) * c.hidden, 256);
+    if (split) {
+      tp.q_lo = tq_lo;
+      tp.scales_lo = ts_lo;
+    }
     rc = launch_gather_quant_mxfp8(tp, stream);
     if (rc) return fail(rc, "MXFP8 activation quant launch failed");
     g_launches += 1;
+    qp.q_lo = qp.scales_lo = nullptr;
+    if (split) {
+      MxQuantParams lp = qp;
+      lp.q = xq_lo;
+      lp.scales = xs_lo;
+      lp.q_in = tq_lo;
+      lp.scales_in = ts_lo;
+      rc = launch_gather_quant_mxfp8(lp, stream);
+      if (rc) return fail(rc, "activation gather launch failed");
+      g_launches += 1;
+    }
     qp.q_in = tq;
     qp.scales_in = ts;
   }

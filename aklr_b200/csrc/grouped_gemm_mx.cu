@@ -751,7 +751,7 @@ __global__ void __launch_bounds__(256) gather_rows_mxfp8_kernel(MxQuantParams p)
 
 int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream) {
   if (p.hidden % 128 != 0) return AKLR_ERR_UNSUPPORTED_SHAPE;
-  if ((p.q_lo != nullptr) != (p.scales_lo != nullptr) || (p.q_lo && (p.q_in || p.row_major_scales || p.act_fp4))) return AKLR_ERR_BAD_ARGUMENT;
+  if ((p.q_lo != nullptr) != (p.scales_lo != nullptr) || (p.q_lo && (p.q_in || p.act_fp4))) return AKLR_ERR_BAD_ARGUMENT;
   if (p.n_rows == 0) return AKLR_OK;
   if (p.q_in) {
     if (!p.sorted_ids || !p.scales_in) return AKLR_ERR_BAD_ARGUMENT;
