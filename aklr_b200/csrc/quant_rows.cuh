@@ -55,63 +55,82 @@ struct ExactDivider {
   }
 };
 
-// One half-warp (16 lanes x 8 values) per 1 x 128 group: this half-warp takes groups ``first``,
-// ``first + stride``, ... of the row table (the caller's grid-stride, or one CTA's share), kGroupsInFlight of
-// them at a time.
-constexpr int kGroupsInFlight = 1;  // measured on the layer's quantiser: 1 -> 0.121 ms, 2 -> 0.125, 4 -> 0.133 (T = 4096)
-constexpr int kOpGroupsInFlight = 1;  // the standalone quantisers: 1 -> 75.8 us, 2 and 4 -> 81.9 us (16384 x 7168)
+// Eight lanes x 16 consecutive values per 1 x 128 group, two 16-byte loads and one 16-byte store per lane.  Once the
+// loads are wide these passes are bound by instructions, not by bytes: a group's reduction and its two true divisions
+// cost the same whatever a lane holds, so 16 lanes x 8 values paid them twice (once per token at 16384 x 7168: 120 -> 90 us, the
+// stand-alone op at 2048 x 7168 10.4 -> 8.5).
+constexpr int kGroupLanes = 8;
 
+struct GroupValues {
+  float v[16];
+  __device__ __forceinline__ void load(const uint16_t* __restrict__ x) {  // this lane's 16 values
+    const uint4 lo = *reinterpret_cast<const uint4*>(x), hi = *reinterpret_cast<const uint4*>(x + 8);
+    const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+  }
+  __device__ __forceinline__ float group_amax(uint32_t group_mask) const {
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(v[i]));
+#pragma unroll
+    for (int off = kGroupLanes / 2; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(group_mask, m, off, kGroupLanes));
+    return m;
+  }
+  // 16 bytes in one store where the caller's buffer allows it (``wide``; eight-byte alignment is all that is asked of it)
+  static __device__ __forceinline__ void store(uint8_t* dst, const uint4& codes, bool wide) {
+    if (wide) {
+      *reinterpret_cast<uint4*>(dst) = codes;
+    } else {
+      reinterpret_cast<uint2*>(dst)[0] = make_uint2(codes.x, codes.y);
+      reinterpret_cast<uint2*>(dst)[1] = make_uint2(codes.z, codes.w);
+    }
+  }
+  __device__ __forceinline__ uint4 pack() const {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = cvt_e4m3x2(v[4 * i], v[4 * i + 1]) | (static_cast<uint32_t>(cvt_e4m3x2(v[4 * i + 2], v[4 * i + 3])) << 16);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+
+// This group of eight lanes takes groups ``first``, ``first + stride``, ... of the row table (the caller's grid-stride).
 __device__ __forceinline__ void gather_quant_fp8_groups(const GatherQuantParams& p, int64_t first, int64_t stride) {
   const int groups_per_row = p.hidden >> 7;
   const int n_rows = p.num_rows ? min(*p.num_rows, p.n_rows) : p.n_rows;
   const int64_t total = static_cast<int64_t>(n_rows) * groups_per_row;
-  const int sub = threadIdx.x & 15;
-  const uint32_t group_mask = 0xFFFFu << (threadIdx.x & 16);  // the lanes of this half-warp
-  for (int64_t g0 = first; g0 < total; g0 += stride * kGroupsInFlight) {
-    uint4 raw[kGroupsInFlight];
-    int row[kGroupsInFlight], grp[kGroupsInFlight];
-    bool live[kGroupsInFlight];
-#pragma unroll
-    for (int u = 0; u < kGroupsInFlight; ++u) {
-      const int64_t g = g0 + u * stride;
-      live[u] = g < total;
-      row[u] = grp[u] = 0;
-      if (live[u]) {
-        // 32-bit division: a 64-bit one is a subroutine of a hundred instructions, per group and lane
-        row[u] = static_cast<int>(static_cast<uint32_t>(g) / static_cast<uint32_t>(groups_per_row));
-        grp[u] = static_cast<int>(static_cast<uint32_t>(g) - static_cast<uint32_t>(row[u]) * static_cast<uint32_t>(groups_per_row));
-        int token = row[u];
-        if (p.sorted_ids) {
-          const int rid = p.sorted_ids[row[u]];
-          token = rid < 0 ? -1 : rid / p.routes_per_token;
-        }
-        live[u] = token >= 0;  // padding rows are never read back
-        if (!live[u] && p.zero_padding)  // but multiplied: zero codes cost the tensor core least
-          *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(row[u]) * p.hidden + grp[u] * 128 + sub * 8) = make_uint2(0u, 0u);
-        if (live[u])
-          raw[u] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.x) +
-                                                   static_cast<size_t>(token) * p.hidden + grp[u] * 128 + sub * 8);
-      }
+  const int sub = threadIdx.x & (kGroupLanes - 1);
+  const uint32_t group_mask = 0xFFu << (threadIdx.x & 24);
+  const bool wide = reinterpret_cast<uintptr_t>(p.q) % 16 == 0;
+  for (int64_t g = first; g < total; g += stride) {
+    // 32-bit division: a 64-bit one is a subroutine of a hundred instructions, per group and lane
+    const int row = static_cast<int>(static_cast<uint32_t>(g) / static_cast<uint32_t>(groups_per_row));
+    const int grp = static_cast<int>(static_cast<uint32_t>(g) - static_cast<uint32_t>(row) * static_cast<uint32_t>(groups_per_row));
+    int token = row;
+    if (p.sorted_ids) {
+      const int rid = p.sorted_ids[row];
+      token = rid < 0 ? -1 : rid / p.routes_per_token;
     }
+    uint8_t* dst = p.q + static_cast<size_t>(row) * p.hidden + grp * 128 + sub * 16;
+    if (token < 0) {  // padding rows are never read back; uniform over the group's lanes
+      if (p.zero_padding) GroupValues::store(dst, make_uint4(0u, 0u, 0u, 0u), wide);  // but multiplied: zero codes cost the tensor core least
+      continue;
+    }
+    GroupValues x;
+    x.load(reinterpret_cast<const uint16_t*>(p.x) + static_cast<size_t>(token) * p.hidden + grp * 128 + sub * 16);
+    const float scale = fmaxf(__fdiv_rn(x.group_amax(group_mask), 448.0f), FLT_MIN);
+    const ExactDivider divide(scale);
 #pragma unroll
-    for (int u = 0; u < kGroupsInFlight; ++u) {
-      if (!live[u]) continue;  // uniform over the half-warp: all of its lanes work on the same group
-      float v[8];
-      unpack8(raw[u], v);
-      float m = amax8(v);
-#pragma unroll
-      for (int off = 8; off >= 1; off >>= 1) m = fmaxf(m, __shfl_xor_sync(group_mask, m, off, 16));
-      const float scale = fmaxf(__fdiv_rn(m, 448.0f), FLT_MIN);
-      const ExactDivider divide(scale);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = divide(v[i]);
-      *reinterpret_cast<uint2*>(p.q + static_cast<size_t>(row[u]) * p.hidden + grp[u] * 128 + sub * 8) = pack8_e4m3(v);
-      if (sub == 0) {
-        if (p.block_m > 0)  // [block][group][row in block]: what the grouped GEMM stages per tile
-          p.scales[(static_cast<size_t>(row[u] / p.block_m) * groups_per_row + grp[u]) * p.block_m + row[u] % p.block_m] = scale;
-        else
-          p.scales[static_cast<size_t>(row[u]) * groups_per_row + grp[u]] = scale;
-      }
+    for (int i = 0; i < 16; ++i) x.v[i] = divide(x.v[i]);
+    GroupValues::store(dst, x.pack(), wide);
+    if (sub == 0) {
+      if (p.block_m > 0)  // [block][group][row in block]: what the grouped GEMM stages per tile
+        p.scales[(static_cast<size_t>(row / p.block_m) * groups_per_row + grp) * p.block_m + row % p.block_m] = scale;
+      else
+        p.scales[static_cast<size_t>(row) * groups_per_row + grp] = scale;
     }
   }
 }
