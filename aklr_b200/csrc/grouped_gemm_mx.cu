@@ -64,7 +64,7 @@ __host__ __device__ inline MxLayout mx_layout(int stages, bool gate_up, bool spl
   l.off_rid = l.off_out + (gate_up ? 0 : (kEpi / 32) * 32 * kOutPassCols * 2);
   l.off_wgt = l.off_rid + kBM * 4;
   l.off_bars = l.off_wgt + kBM * 4;
-  l.total = l.off_bars + (3 * stages + 2) * 8 + 16;
+  l.total = l.off_bars + (2 * stages + 2) * 8 + 16;
   return l;
 }
 
@@ -190,8 +190,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
   float* wgt_s = reinterpret_cast<float*>(smem + L.off_wgt);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.off_bars);
   uint64_t* empty = full + S;
-  uint64_t* sf_full = empty + S;
-  uint64_t* acc_full = sf_full + S;
+  uint64_t* acc_full = empty + S;
   uint64_t* acc_empty = acc_full + 1;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
@@ -199,9 +198,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], 2);  // the producer's announcement and the staging warp that owns the K-block
       mbar_init(&empty[s], 1);
-      mbar_init(&sf_full[s], 1);  // the staging warp that owns the K-block
     }
     mbar_init(acc_full, 1);
     mbar_init(acc_empty, kEpi / 32);
@@ -299,7 +297,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
       if (!mbar_wait_warp(acc_empty, (tile_no & 1) ^ 1, abort_flag, p.status, 22)) break;
       for (int kb = 0; kb < KB; ++kb) {
         if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 23)) { ok = false; break; }
-        if (!mbar_wait_warp(&sf_full[s], ph, abort_flag, p.status, 24)) { ok = false; break; }
         tc_fence_after_sync();
         if (leader) {
           const uint64_t sfa = sfa0 + step;
@@ -390,7 +387,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
             *reinterpret_cast<uint32_t*>(sf + kSfaBytes + (q >> 2) * 512 + lane * 16 + (q & 3) * 4) = wq[d][q];
           fence_proxy_async_smem();  // tcgen05.cp reads these bytes through the async proxy
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sf_full[s]);
+          if (lane == 0) mbar_arrive(&full[s]);
           s += 2;
           if (s >= S) { s -= S; ph ^= 1; }
           load(wq[d], aq[d], aq_lo[SPLIT ? d : 0]);
@@ -575,6 +572,15 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
           continue;
         }
         uint8_t* stage = smem + L.off_out + (warp - 2) * (32 * kOutPassCols * 2);
+        // where this lane's four rows of a pass go (their route ids sit in the warp's other lanes); null: padding
+        uint8_t* dst[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rr = __shfl_sync(0xFFFFFFFFu, rid, 8 * i + (lane >> 2));
+          dst[i] = rr < 0 || bad ? nullptr
+                                 : static_cast<uint8_t*>(p.out_rows) +
+                                       (static_cast<size_t>(rr) * p.out_dim + j * 256 + half * 128 + (lane & 3) * 8) * 2;
+        }
 #pragma unroll
         for (int pass = 0; pass < 128 / kOutPassCols; ++pass) {
 #pragma unroll
@@ -590,16 +596,15 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
                 make_uint4(o[0], o[1], o[2], o[3]);
           }
           __syncwarp();
+          uint4 val[4];  // all of a pass's reads before its first store: nothing waits for a read but its own store
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int r = 8 * i + (lane >> 2), c = lane & 3;  // row of this warp's 32, 16-byte chunk
-            const int rr = rid_s[quarter * 32 + r];
-            const uint4 val = *reinterpret_cast<const uint4*>(stage + r * (kOutPassCols * 2) + ((c ^ ((r >> 1) & 3)) << 4));
-            if (rr >= 0 && !bad)
-              *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out_rows) +
-                                        (static_cast<size_t>(rr) * p.out_dim + j * 256 + half * 128 +
-                                         pass * kOutPassCols + c * 8) * 2) = val;
+            val[i] = *reinterpret_cast<const uint4*>(stage + r * (kOutPassCols * 2) + ((c ^ ((r >> 1) & 3)) << 4));
           }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (dst[i]) *reinterpret_cast<uint4*>(dst[i] + pass * (kOutPassCols * 2)) = val[i];
           __syncwarp();
         }
       }
