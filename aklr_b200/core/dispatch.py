@@ -193,6 +193,23 @@ class CallRecorder:
         return path
 
 
+def _binder(signature: inspect.Signature, name: str) -> Callable[..., dict]:
+    """A function of exactly ``signature``'s parameters that returns them as a dict, defaults filled in.
+
+    The interpreter binds a call's arguments to it in well under a microsecond; ``Signature.bind`` walks them in Python
+    and takes 5-10, which a decode call of a small layer waits for (its kernels are launched as fast as the host calls)."""
+    defaults = {f"_default_{p.name}": p.default for p in signature.parameters.values() if p.default is not p.empty}
+    parameters = []
+    for p in signature.parameters.values():
+        if p.kind is not p.POSITIONAL_OR_KEYWORD:
+            raise TypeError(f"{name}: parameter {p.name} must be an ordinary one")
+        parameters.append(p.name + (f"=_default_{p.name}" if p.default is not p.empty else ""))
+    items = ", ".join(f"{p!r}: {p}" for p in signature.parameters)
+    namespace = dict(defaults)
+    exec(f"def {name}({', '.join(parameters)}):\n    return {{{items}}}", namespace)
+    return namespace[name]
+
+
 @dataclass
 class KernelDispatcher:
     """Serves one contract.  Closed (every call returns ``closed_reason``) until the registry opens
@@ -276,19 +293,16 @@ class KernelDispatcher:
         self.contract.check_api_signature(fn)
         signature = inspect.signature(fn)
 
-        def bind(args, kwargs) -> dict:
-            bound = signature.bind(*args, **kwargs)
-            bound.apply_defaults()
-            return dict(bound.arguments)
+        bind = _binder(signature, fn.__name__)
 
         def api_fn(*args, **kwargs):
-            return self.dispatch(bind(args, kwargs))
+            return self.dispatch(bind(*args, **kwargs))
 
         def fallback_reason(*args, **kwargs):
-            return self.fallback_reason(bind(args, kwargs))
+            return self.fallback_reason(bind(*args, **kwargs))
 
         def serving(*args, **kwargs):
-            return self.serving(bind(args, kwargs))
+            return self.serving(bind(*args, **kwargs))
 
         for generated in (api_fn, fallback_reason, serving):
             generated.__name__ = fn.__name__

@@ -165,7 +165,7 @@ class CudaKernels:
             _lib.check(
                 lib.aklr_moe_mxfp4_experts_rows(
                     ctypes.byref(cfg), base, layout.row_bytes, base + h, layout.row_bytes, _ptr(ids), _ptr(weights), _ptr(w1), _ptr(s1),
-                    _ptr(w2), _ptr(s2), float(self.swiglu_limit or 0.0), _ptr(out), ws.base.data_ptr(), ws.layout.total_bytes, _stream(),
+                    _ptr(w2), _ptr(s2), float(self.swiglu_limit or 0.0), _ptr(out), ws.base_ptr, ws.layout.total_bytes, _stream(),
                 )
             )
             return out
@@ -174,7 +174,7 @@ class CudaKernels:
         _lib.check(
             lib.aklr_moe_fp8_experts_rows(
                 ctypes.byref(cfg), base, layout.row_bytes, base + h, layout.row_bytes, _ptr(ids), _ptr(weights), _ptr(w1), _ptr(s1),
-                _ptr(w2), _ptr(s2), _ptr(out), ws.base.data_ptr(), ws.layout.total_bytes, _stream(),
+                _ptr(w2), _ptr(s2), _ptr(out), ws.base_ptr, ws.layout.total_bytes, _stream(),
             )
         )
         return out

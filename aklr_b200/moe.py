@@ -19,7 +19,8 @@ _SIGMOID_TABLES: dict[torch.device, torch.Tensor] = {}
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the current stream's handle without a Stream object around it: 0.2 us instead of 1.5
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -109,8 +110,15 @@ class Workspace:
         self.cfg = cfg
         self.layout = workspace_layout(cfg)
         self.buffer = torch.empty(self.layout.total_bytes + 1024, dtype=torch.uint8, device=device)
-        shift = (-self.buffer.data_ptr()) % 1024
-        self.base = self.buffer[shift : shift + self.layout.total_bytes]
+        self.shift = (-self.buffer.data_ptr()) % 1024
+
+    @property
+    def base(self) -> torch.Tensor:
+        return self.buffer[self.shift : self.shift + self.layout.total_bytes]
+
+    @property
+    def base_ptr(self) -> int:
+        return self.buffer.data_ptr() + self.shift
 
     def _view(self, offset: int, count: int, dtype: torch.dtype) -> torch.Tensor:
         size = torch.empty((), dtype=dtype).element_size()
@@ -119,7 +127,7 @@ class Workspace:
     def check_status(self) -> None:
         """Waits for the stream and raises if a device-side wait gave up."""
         status = (ctypes.c_int32 * 2)()
-        _lib.check(_lib.load().aklr_moe_read_status(self.base.data_ptr(), status, _stream()))
+        _lib.check(_lib.load().aklr_moe_read_status(self.base_ptr, status, _stream()))
 
     @property
     def routes_per_token(self) -> int:
@@ -231,7 +239,7 @@ def fused_moe_fp8(
             _ptr(w2),
             _ptr(w2_scale),
             _ptr(out),
-            ws.base.data_ptr(),
+            ws.base_ptr,
             ws.layout.total_bytes,
             _stream(),
         )
@@ -276,7 +284,7 @@ def fused_experts_fp8(
             _ptr(w2),
             _ptr(w2_scale),
             _ptr(out),
-            ws.base.data_ptr(),
+            ws.base_ptr,
             ws.layout.total_bytes,
             _stream(),
         )
@@ -354,7 +362,7 @@ def fused_experts_mxfp4(
     _lib.check(
         _lib.load().aklr_moe_mxfp4_experts_ex(
             ctypes.byref(cfg), _ptr(hidden_states), _ptr(topk_ids), _ptr(topk_weights), _ptr(expert_map), _ptr(w1),
-            _ptr(w1_scale), _ptr(w2), _ptr(w2_scale), ctypes.byref(options), _ptr(out), ws.base.data_ptr(),
+            _ptr(w1_scale), _ptr(w2), _ptr(w2_scale), ctypes.byref(options), _ptr(out), ws.base_ptr,
             ws.layout.total_bytes, _stream(),
         )
     )
@@ -392,7 +400,7 @@ def fused_moe_mxfp4(
     _lib.check(
         _lib.load().aklr_moe_mxfp4_forward(
             ctypes.byref(cfg), _ptr(hidden_states), _ptr(logits), _ptr(bias), _ptr(table), _ptr(w1), _ptr(w1_scale),
-            _ptr(w2), _ptr(w2_scale), float(swiglu_limit or 0.0), _ptr(out), ws.base.data_ptr(), ws.layout.total_bytes,
+            _ptr(w2), _ptr(w2_scale), float(swiglu_limit or 0.0), _ptr(out), ws.base_ptr, ws.layout.total_bytes,
             _stream(),
         )
     )
