@@ -423,6 +423,12 @@ __device__ int block_exclusive_scan(int v, int* scratch, int* total) {
   return inc - v + (warp > 0 ? scratch[warp - 1] : 0);
 }
 
+// -1 in the padding rows: from this block size on a warp per expert writes them (one thread per expert stores up to 127 of
+// them one after the other: 64 tokens on 257 experts in 128-row blocks, 21 -> 9 us for the sort with place_chunk's table).
+// Below it the thread that plans an expert does: 15 or 31 stores at most, and a decode call finds the code in its caches
+// (one token: 84.9 us for the call, 86.7 with the warps).
+constexpr int kWarpFillBlock = 64;
+
 // Shared by the scan kernel and the one-CTA path: from per-expert totals in smem ``total`` compute
 // padded bases, the block table, counts, the pad fill.  ``base`` receives each expert's first row.
 __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, int* scratch) {
@@ -467,16 +473,30 @@ __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, i
         for (int b = 0; b < nb; b += 2)
           p.pair_table[pair_running++] = (running + b) | (b + 1 < nb ? static_cast<int>(0x80000000u) : 0);
       }
-      for (int r = c; r < nb * p.block_m; ++r) p.sorted_ids[running * p.block_m + r] = -1;
+      if (p.block_m < kWarpFillBlock)
+        for (int r = c; r < nb * p.block_m; ++r) p.sorted_ids[running * p.block_m + r] = -1;
       running += nb;
     }
+  }
+  __syncthreads();
+  if (p.block_m < kWarpFillBlock) return;
+  for (int e = tid >> 5; e < p.n_experts; e += nt >> 5) {
+    const int c = total[e], end = (c + p.block_m - 1) / p.block_m * p.block_m;
+    for (int r = c + (tid & 31); r < end; r += 32) p.sorted_ids[base[e] + r] = -1;
   }
   __syncthreads();
 }
 
 // Stable placement of one chunk: thread t holds route chunk_start + t.  ``cursor[e]`` is the next
-// free row of expert e for this chunk (smem, updated in warp order so the order stays stable).
-__device__ void place_chunk(const AlignParams& p, int route, int* cursor) {
+// free row of expert e for this chunk (smem, updated so that the order stays stable).
+// ``warp_counts`` [32][n_experts] (smem): how many routes of the chunk each warp has for each expert; one thread per
+// expert then sums over the warps, and the chunk takes four barriers.  Without the table -- null, where the expert counts do
+// not fit, and chunks of at most kSerialWarps warps -- the warps take their rows one after the other, a barrier each:
+// 333 tokens x 8 routes, three chunks in one CTA, 19.6 us that way, 13.2 by the table; 17 tokens x 11 routes (six warps, 513
+// experts) 83.1 us for the call that way, 86.4 by the table.
+constexpr int kSerialWarps = 8;
+constexpr int kWarpCountExperts = 544;  // 32 x 544 counts and the int arrays stay under the 48 KB a launch gets unasked
+__device__ void place_chunk(const AlignParams& p, int route, int* cursor, uint16_t* warp_counts) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e = route < p.n_routes ? local_expert(p, route) : -1;
   const uint32_t active = __ballot_sync(0xFFFFFFFFu, e >= 0);
@@ -489,6 +509,26 @@ __device__ void place_chunk(const AlignParams& p, int route, int* cursor) {
   const int in_chunk = p.n_routes - chunk_first < static_cast<int>(blockDim.x) ? p.n_routes - chunk_first
                                                                                 : static_cast<int>(blockDim.x);
   const int busy_warps = in_chunk > 0 ? (in_chunk + 31) >> 5 : 0;  // warps past these hold no route
+  if (warp_counts && busy_warps > kSerialWarps) {
+    for (int i = threadIdx.x; i < busy_warps * p.n_experts; i += blockDim.x) warp_counts[i] = 0;
+    __syncthreads();
+    if (leader) warp_counts[warp * p.n_experts + e] = static_cast<uint16_t>(__popc(same));
+    __syncthreads();
+    int chunk_total = 0;  // thread i < n_experts: expert i's routes in this chunk (n_experts <= blockDim.x)
+    if (static_cast<int>(threadIdx.x) < p.n_experts) {
+#pragma unroll 8
+      for (int w = 0; w < busy_warps; ++w) {
+        const int c = warp_counts[w * p.n_experts + threadIdx.x];
+        warp_counts[w * p.n_experts + threadIdx.x] = static_cast<uint16_t>(chunk_total);
+        chunk_total += c;
+      }
+    }
+    __syncthreads();
+    if (e >= 0) p.sorted_ids[cursor[e] + warp_counts[warp * p.n_experts + e] + rank_in_warp] = route;
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < p.n_experts) cursor[threadIdx.x] += chunk_total;
+    return;  // the caller's barrier, or the end of the kernel, follows
+  }
   for (int w = 0; w < busy_warps; ++w) {
     if (warp == w && leader) {
       start = cursor[e];
@@ -500,6 +540,14 @@ __device__ void place_chunk(const AlignParams& p, int route, int* cursor) {
     start = __shfl_sync(same, start, __ffs(same) - 1);
     p.sorted_ids[start + rank_in_warp] = route;
   }
+}
+
+// The table behind the int arrays of a sort kernel's shared memory, where the launch made room for it.
+__host__ __device__ inline size_t warp_count_bytes(int n_experts) {
+  return n_experts <= kWarpCountExperts ? static_cast<size_t>(32) * n_experts * sizeof(uint16_t) : 0;
+}
+__device__ __forceinline__ uint16_t* warp_count_table(const AlignParams& p, int* after) {
+  return warp_count_bytes(p.n_experts) ? reinterpret_cast<uint16_t*>(after) : nullptr;
 }
 
 // Pass 2 (one CTA): per-expert totals, per-chunk offsets, block table.
@@ -552,12 +600,12 @@ __global__ void __launch_bounds__(kSortChunk) align_scatter_kernel(AlignParams p
   for (int e = threadIdx.x; e < p.n_experts; e += blockDim.x)
     cursor[e] = p.chunk_hist[static_cast<size_t>(blockIdx.x) * p.n_experts + e];
   __syncthreads();
-  place_chunk(p, blockIdx.x * kSortChunk + threadIdx.x, cursor);
+  place_chunk(p, blockIdx.x * kSortChunk + threadIdx.x, cursor, warp_count_table(p, cursor + p.n_experts));
 }
 
 // All three passes in one CTA, for up to kSmallRoutes routes (decode batches).
 constexpr int kSmallRoutes = 4096;
-__device__ void align_small_body(const AlignParams& p, int* sm) {
+__device__ void align_small_body(const AlignParams& p, int* sm, bool with_table) {
   int* total = sm;
   int* base = sm + p.n_experts;
   int* scratch = base + p.n_experts;
@@ -570,7 +618,7 @@ __device__ void align_small_body(const AlignParams& p, int* sm) {
   __syncthreads();
   plan_blocks(p, total, base, scratch);
   for (int start = 0; start < p.n_routes; start += blockDim.x) {  // a chunk is one route per thread
-    place_chunk(p, start + threadIdx.x, base);
+    place_chunk(p, start + threadIdx.x, base, with_table ? warp_count_table(p, scratch + 1024) : nullptr);
     __syncthreads();
   }
 }
@@ -579,7 +627,7 @@ __global__ void __launch_bounds__(kSortChunk) align_small_kernel(AlignParams p) 
   extern __shared__ int sm[];
   griddep_wait();
   griddep_launch();
-  align_small_body(p, sm);
+  align_small_body(p, sm, true);
 }
 
 // Routing and sort of a decode call in one CTA: route each token by counting, then sort the routes
@@ -615,7 +663,7 @@ __global__ void __launch_bounds__(kSortChunk) decode_prologue_kernel(RouteParams
       route_by_counting(rp, token, e, kDecodePrologueExperts, 1 + team, s[r], image[r], sh[team]);
   }
   __syncthreads();  // every token's ids are written
-  align_small_body(ap, sm);
+  align_small_body(ap, sm, false);  // at most kDecodePrologueTokens tokens: a few warps of routes
 }
 
 int launch_decode_prologue(const RouteParams& rp, const AlignParams& ap, cudaStream_t stream) {
@@ -635,13 +683,14 @@ int launch_align(const AlignParams& p, cudaStream_t stream) {
   const size_t smem = (2 * static_cast<size_t>(p.n_experts) + 1024) * sizeof(int);
   cudaError_t err = cudaSuccess;
   if (p.n_routes <= kSmallRoutes) {
-    err = launch_kernel(align_small_kernel, dim3(1), dim3(kSortChunk), smem, stream, 1, p);
+    err = launch_kernel(align_small_kernel, dim3(1), dim3(kSortChunk), smem + warp_count_bytes(p.n_experts), stream, 1, p);
   } else {
     const int chunks = (p.n_routes + kSortChunk - 1) / kSortChunk;
     err = launch_kernel(align_count_kernel, dim3(chunks), dim3(kSortChunk), p.n_experts * sizeof(int), stream, 1, p);
     if (err == cudaSuccess) err = launch_kernel(align_scan_kernel, dim3(1), dim3(1024), smem, stream, 1, p, chunks);
     if (err == cudaSuccess)
-      err = launch_kernel(align_scatter_kernel, dim3(chunks), dim3(kSortChunk), p.n_experts * sizeof(int), stream, 1, p);
+      err = launch_kernel(align_scatter_kernel, dim3(chunks), dim3(kSortChunk), p.n_experts * sizeof(int) + warp_count_bytes(p.n_experts),
+                          stream, 1, p);
   }
   return err == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }

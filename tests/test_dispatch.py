@@ -245,3 +245,24 @@ def test_tile_contiguous_layout_round_trips_on_the_host():
 
     with pytest.raises(ValueError, match="CUDA"):
         layouts.to_b200_tiled(w)
+
+
+def test_api_arguments_bind_as_their_signature_does():
+    """The generated binder against ``inspect.Signature.bind``: every form a call can take, and the ones it cannot."""
+    import inspect
+
+    from aklr_b200.core.dispatch import _binder
+
+    def fn(a, b, c=3, d=None): ...
+
+    signature = inspect.signature(fn)
+    bind = _binder(signature, "fn")
+    for args, kwargs in (((1, 2), {}), ((1,), {"b": 5}), ((), {"d": 1, "b": 2, "a": 0}), ((1, 2, 3, 4), {}), ((1, 2), {"c": None})):
+        want = signature.bind(*args, **kwargs)
+        want.apply_defaults()
+        assert bind(*args, **kwargs) == dict(want.arguments) and list(bind(*args, **kwargs)) == list(want.arguments)
+    for args, kwargs in (((1,), {}), ((1, 2, 3, 4, 5), {}), ((1, 2), {"e": 1}), ((1, 2), {"a": 1})):
+        with pytest.raises(TypeError):
+            signature.bind(*args, **kwargs)
+        with pytest.raises(TypeError):
+            bind(*args, **kwargs)

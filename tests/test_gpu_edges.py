@@ -1,0 +1,115 @@
+"""The edges of the kernels whose tiles, boxes and tables depend on the call's sizes."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from aklr_b200 import workloads as wl
+from oracle import moe_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def dev():
+    return torch.device("cuda:0")
+
+
+def router_case(tokens, hidden, experts, dtype):
+    g = torch.Generator().manual_seed(tokens * 1000 + hidden + experts)
+    x = torch.randn(tokens, hidden, generator=g).to(torch.bfloat16)
+    w = (torch.randn(experts, hidden, generator=g) * hidden**-0.5).to(dtype)
+    exact = x.double() @ w.double().T
+    return x, w, exact, x.double().abs() @ w.double().abs().T
+
+
+@pytest.mark.parametrize("tokens", [1, 2, 3, 16, 17, 63, 64, 129])
+@pytest.mark.parametrize("hidden,experts", [(136, 7), (192, 33), (2048, 512), (7168, 256)])
+def test_bf16_router_at_every_shape_of_its_kernels(tokens, hidden, experts):
+    """One token, 2 x 2 and 2 x 4 dot products per warp, the tensor-core tiles with one and two boxes of K per stage.
+    Bound: the rounding to bf16 (2^-8 of the value) and at most 2^-23 of the sum of magnitudes for every 16th of the chain."""
+    from aklr_b200.moe import router_logits
+
+    if hidden % 64 and tokens >= 64:
+        pytest.skip("the tensor-core kernel needs whole boxes of K: such a call takes the dot products tested below 64 tokens")
+    x, w, exact, magnitude = router_case(tokens, hidden, experts, torch.bfloat16)
+    got = router_logits(x.to(dev()), w.to(dev())).cpu().double()
+    assert ((got - exact).abs() <= 2.0**-8 * exact.abs() + (hidden / 16 + 16) * 2.0**-23 * magnitude).all()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 128, 129, 300])
+@pytest.mark.parametrize("hidden,experts", [(128, 1), (384, 33), (768, 40), (3072, 256)])
+def test_float32_router_keeps_float32_accuracy(tokens, hidden, experts):
+    """Dot products up to 16 tokens, three bf16 terms on the tensor cores from 17; fewer K steps than accumulators (128),
+    ragged expert tiles.  Bound: a truncation of 2^-23 of the partial sum, itself at most the sum of magnitudes, per
+    16 products, and the final additions."""
+    from aklr_b200.moe import router_logits_f32
+
+    x, w, exact, magnitude = router_case(tokens, hidden, experts, torch.float32)
+    got = router_logits_f32(x.to(dev()), w.to(dev())).cpu().double()
+    assert ((got - exact).abs() <= (hidden / 16 + 32) * 2.0**-23 * magnitude).all()
+    if tokens > 16:  # token rows at 8-byte alignment cannot be a TMA operand: the CUDA-core tile serves them
+        shifted = torch.empty(x.numel() + 4, dtype=torch.bfloat16, device=dev())[4:].view(x.shape)
+        shifted.copy_(x)
+        again = router_logits_f32(shifted, w.to(dev())).cpu().double()
+        assert ((again - exact).abs() <= (hidden + 32) * 2.0**-24 * magnitude).all()
+
+
+@pytest.mark.parametrize("n_experts", [1, 31, 543, 544, 545, 1025])
+@pytest.mark.parametrize("n_tokens,k,block_m", [(1, 1, 16), (33, 1, 128), (1025, 1, 16), (4096, 1, 32), (4097, 1, 128)])
+def test_sort_with_and_without_the_per_warp_counts(n_experts, n_tokens, k, block_m):
+    """The per-warp count table serves up to 544 experts; one CTA up to 4096 routes, chunks of 1024 beyond."""
+    from aklr_b200.moe import moe_align
+
+    g = torch.Generator().manual_seed(n_experts + n_tokens)
+    ids = torch.randint(0, n_experts, (n_tokens, k), generator=g).to(torch.int32)
+    sorted_ids, block_expert, counts, nb = moe_align(ids.to(dev()), n_experts, block_m)
+    ref_sorted, ref_blocks, ref_counts = orc.moe_align(ids, n_experts, block_m)
+    assert torch.equal(counts.cpu().long(), ref_counts) and nb == ref_blocks.numel()
+    assert torch.equal(block_expert.cpu(), ref_blocks)
+    assert torch.equal(sorted_ids.cpu(), ref_sorted)
+
+
+@pytest.mark.parametrize("inter", [128, 256, 384])
+@pytest.mark.parametrize("act_bits", [4, 8, 16])
+@pytest.mark.parametrize("copies", [1, 3])
+def test_mxfp4_boxes_at_their_edges(inter, act_bits, copies):
+    """Experts with 1, 8, 9, 16, 17, ... routed rows (boxes of 16, 32, 64 and 128 rows, direct and staged output rows, warps
+    without a row): bit for bit the output of loading all 128 rows, and the oracle's within its gates.  Three routes per
+    token and more than 512 tokens: quantised once per token, then copied."""
+    from aklr_b200 import _lib
+    from aklr_b200.moe import fused_experts_mxfp4
+
+    rows = [1, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129]
+    cfg = wl.MoEConfig("mx", hidden=256, inter=inter, n_routed=len(rows) + 1, topk=1)
+    weights = [t.to(dev()) for t in wl.mx_expert_weights(cfg, 5)]
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(rows)])  # the last expert gets none
+    g = torch.Generator().manual_seed(inter + act_bits)
+    ids = ids[torch.randperm(ids.numel(), generator=g)].view(-1, 1)
+    ids = torch.cat([(ids + 5 * c) % len(rows) for c in range(copies)], dim=1).contiguous()
+    x = torch.randn(ids.shape[0], 256, generator=g).to(torch.bfloat16)
+    route_weights = torch.rand(ids.shape, generator=g)
+    outs = []
+    for variant in (0, _lib.VARIANT_FULL_ACTIVATION_BOXES):
+        out, ws = fused_experts_mxfp4(x.to(dev()), ids.to(dev()), route_weights.to(dev()), *weights, return_workspace=True,
+                                      variant=variant, act_bits=act_bits)
+        ws.check_status()
+        outs.append(out.cpu())
+    assert torch.equal(outs[0], outs[1])
+    ref = orc.mx_experts(x, ids.long(), route_weights, *[t.cpu() for t in weights], act_bits=act_bits)
+    gates = orc.output_gates(outs[0], ref)
+    assert orc.gates_pass(gates, min_sqnr_db=30.0 if act_bits != 4 else 20.0), gates
+
+
+@pytest.mark.parametrize("rows,hidden", [(1, 128), (37, 384), (600, 7168)])
+def test_quantised_codes_do_not_depend_on_the_outputs_alignment(rows, hidden):
+    """Sixteen codes in one store where the buffer is 16-byte aligned, in two where it is only 8-byte aligned."""
+    from aklr_b200.moe import per_group_quant_fp8
+
+    x = torch.randn(rows, hidden, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).to(dev())
+    codes, scales = per_group_quant_fp8(x)
+    shifted = torch.empty(rows * hidden + 8, dtype=torch.uint8, device=dev())[8:].view(torch.float8_e4m3fn).view(rows, hidden)
+    codes8, scales8 = per_group_quant_fp8(x, quantized=shifted)
+    assert torch.equal(codes.view(torch.uint8), codes8.view(torch.uint8)) and torch.equal(scales, scales8)
+    amax = x.float().cpu().view(rows, hidden // 128, 128).abs().amax(-1)
+    assert torch.equal(scales.cpu(), (amax.clamp_min(1e-10) * torch.tensor(1.0 / 448.0)).T.contiguous())
