@@ -14,68 +14,74 @@
 
 namespace aklr {
 
-__global__ void __launch_bounds__(256) combine_kernel(CombineParams p) {
+// A warp takes ``chunks_per_item`` runs of 256 columns of one token: its routes are looked at once per item, one lane
+// each, and are a bit mask from then on, so that a thread is left with its rows' loads (nine at a time in flight) and
+// additions.  With every thread reading and testing all of its token's ids per 8 columns the pass issued 45 % of its cycles
+// at three CTAs per SM and reached 69 % of the memory's rate (16384 tokens x 9 routes on 7168, 2.35 GB: 490 -> 385 us, 6.1 TB/s).
+constexpr int kCombineSlots = 9;
+__global__ void __launch_bounds__(256, 4) combine_kernel(CombineParams p, int chunks_per_item, int items_per_token) {
   griddep_wait();
   griddep_launch();
-  const int vec_per_row = p.hidden >> 3;  // 8 bf16 per 16-byte vector
-  const int64_t total = static_cast<int64_t>(p.n_tokens) * vec_per_row;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride) {
-    // 32-bit division (the total is far below 2^31): the 64-bit one is a subroutine
-    const int token = static_cast<int>(static_cast<uint32_t>(i) / static_cast<uint32_t>(vec_per_row));
-    const int v = static_cast<int>(static_cast<uint32_t>(i) - static_cast<uint32_t>(token) * static_cast<uint32_t>(vec_per_row));
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const bool received = !p.num_local_tokens || token < __ldg(p.num_local_tokens);
-    // Slots are summed in order, but their loads do not wait for one another: ids of a batch of
-    // slots first, then all of its rows, then the additions (a decode call is one latency chain).
-    constexpr int kBatchSlots = 9;
-    for (int s0 = 0; s0 < p.routes_per_token; s0 += kBatchSlots) {
-      bool live[kBatchSlots];
-      uint4 raw[kBatchSlots];
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const int items = p.n_tokens * items_per_token;  // < 2^31: checked at launch
+  for (int item = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; item < items; item += warps) {
+    const int token = static_cast<int>(static_cast<uint32_t>(item) / static_cast<uint32_t>(items_per_token));
+    const int chunk0 = (item - token * items_per_token) * chunks_per_item;
+    bool mine = false;  // lane s: whether slot s of the token is added here (at most 32 slots)
+    if (lane < p.routes_per_token && (!p.num_local_tokens || token < __ldg(p.num_local_tokens))) {
+      const int e = __ldg(p.topk_ids + token * p.routes_per_token + lane);
+      mine = e >= 0 && e < p.n_experts_global && (!p.expert_map || __ldg(p.expert_map + e) >= 0);
+    }
+    const uint32_t live = __ballot_sync(0xFFFFFFFFu, mine);
+    const uint16_t* rows = static_cast<const uint16_t*>(p.rows) + static_cast<size_t>(token) * p.routes_per_token * p.hidden;
+    uint16_t* out = static_cast<uint16_t*>(p.out) + static_cast<size_t>(token) * p.hidden;
+    for (int c = 0; c < chunks_per_item; ++c) {
+      const int col = (chunk0 + c) * 256 + lane * 8;
+      if (col >= p.hidden) break;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      // slots are summed in order; their loads do not wait for one another
+      for (int s0 = 0; s0 < p.routes_per_token; s0 += kCombineSlots) {
+        uint4 raw[kCombineSlots];
 #pragma unroll
-      for (int d = 0; d < kBatchSlots; ++d) {
-        const int s = s0 + d;
-        live[d] = false;
-        if (s < p.routes_per_token) {
-          const int e = __ldg(p.topk_ids + token * p.routes_per_token + s);
-          live[d] = received && e >= 0 && e < p.n_experts_global && (!p.expert_map || __ldg(p.expert_map + e) >= 0);
+        for (int d = 0; d < kCombineSlots; ++d)
+          if (s0 + d < 32 && (live >> (s0 + d)) & 1u)
+            raw[d] = *reinterpret_cast<const uint4*>(rows + static_cast<size_t>(s0 + d) * p.hidden + col);
+#pragma unroll
+        for (int d = 0; d < kCombineSlots; ++d) {
+          if (s0 + d >= 32 || !((live >> (s0 + d)) & 1u)) continue;
+          const uint32_t w[4] = {raw[d].x, raw[d].y, raw[d].z, raw[d].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[2 * q] += __uint_as_float(w[q] << 16);
+            acc[2 * q + 1] += __uint_as_float(w[q] & 0xFFFF0000u);
+          }
         }
       }
+      uint4 packed;
+      uint32_t* o = reinterpret_cast<uint32_t*>(&packed);
 #pragma unroll
-      for (int d = 0; d < kBatchSlots; ++d)
-        if (live[d])
-          raw[d] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.rows) +
-                                                   static_cast<size_t>(token * p.routes_per_token + s0 + d) * p.hidden + v * 8);
-#pragma unroll
-      for (int d = 0; d < kBatchSlots; ++d) {
-        if (!live[d]) continue;
-        const uint32_t w[4] = {raw[d].x, raw[d].y, raw[d].z, raw[d].w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          acc[2 * q] += __uint_as_float(w[q] << 16);
-          acc[2 * q + 1] += __uint_as_float(w[q] & 0xFFFF0000u);
-        }
+      for (int q = 0; q < 4; ++q) {
+        const __nv_bfloat162 two = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
+        o[q] = *reinterpret_cast<const uint32_t*>(&two);
       }
+      *reinterpret_cast<uint4*>(out + col) = packed;
     }
-    uint4 packed;
-    uint32_t* o = reinterpret_cast<uint32_t*>(&packed);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const __nv_bfloat162 two = __floats2bfloat162_rn(acc[2 * q], acc[2 * q + 1]);
-      o[q] = *reinterpret_cast<const uint32_t*>(&two);
-    }
-    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + static_cast<size_t>(token) * p.hidden + v * 8) = packed;
   }
 }
 
 int launch_combine(const CombineParams& p, cudaStream_t stream) {
-  if (p.hidden % 8 != 0) return AKLR_ERR_UNSUPPORTED_SHAPE;
+  if (p.hidden % 8 != 0 || p.routes_per_token > 32) return AKLR_ERR_UNSUPPORTED_SHAPE;
   if (p.n_tokens == 0) return AKLR_OK;
   const int64_t total = static_cast<int64_t>(p.n_tokens) * (p.hidden / 8);
   if (total >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
-  const int64_t blocks = (total + 255) / 256;
+  // One run per warp until every SM's 32 warps have several; then four, so that an item's look at its routes is shared.
+  const int chunks = (p.hidden + 255) / 256;
+  const int per_item = static_cast<int64_t>(p.n_tokens) * chunks >= 148 * 32 * 8 ? 4 : 1;
+  const int per_token = (chunks + per_item - 1) / per_item;
+  const int64_t blocks = (static_cast<int64_t>(p.n_tokens) * per_token + 7) / 8;
   const int grid = static_cast<int>(blocks < 148 * 8 ? blocks : 148 * 8);
-  return launch_kernel(combine_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  return launch_kernel(combine_kernel, dim3(grid), dim3(256), 0, stream, 1, p, per_item, per_token) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 // One warp per (TOKENS tokens, EXPERTS experts): lanes stride the hidden dimension with 16-byte loads, and the loads of
