@@ -5,10 +5,9 @@
 // equals, the lower expert id -- the order the reference's stable descending sort defines
 // (aklr/plugins/sglang/models/deepseek_v2/reference.py:114-143,
 //  aklr/plugins/sglang/models/qwen3_moe/reference.py:34-41, aklr/ops/topk/reference.py:17-35).
-// Two kernels pick by those keys and give bit-identical tables: large batches take one warp per
-// token (every pick a warp arg-max), batches up to 2048 tokens one CTA per token with one thread per
-// expert that COUNTS the keys greater than its own (no chain of dependent reductions: ~3 us
-// instead of ~15 us for a handful of tokens).  One to eight tokens run routing and sort as one CTA.
+// Two kernels pick by those keys and give bit-identical tables: one warp per token (every pick a warp arg-max), or, for
+// small batches under grouped or sigmoid routing (routes_by_counting), one CTA per token with one thread per
+// expert that COUNTS the keys greater than its own (no chain of dependent reductions).  One to eight tokens run routing and sort as one CTA.
 //
 // Sort: a stable counting sort of routes (token*K + slot) by expert, each expert's run padded
 // with -1 to a multiple of block_m, plus a block -> expert table.  The reference defines no order
@@ -326,8 +325,15 @@ __global__ void __launch_bounds__(1024) route_count_kernel(RouteParams p) {
   route_by_counting(p, blockIdx.x, threadIdx.x, blockDim.x, 0, s, image, sh);
 }
 
-// Batches up to this many tokens are routed by counting (one CTA per token).
-constexpr int kCountingRouteTokens = 2048;
+// Whether a batch is routed by counting (one CTA per token) or by warp arg-maxes.  A count compares every key with every
+// other of its group: short for grouped routing, E * E per token without groups.  Microseconds per launch, counting / warps,
+// at 64, 512 and 2048 tokens: grouped 256 experts 3.1 / 9.7, 5.9 / 10.0, 13.6 / 12.8; sigmoid 256 experts without groups
+// 4.3 / 5.9, 9.7 / 6.1, 28.7 / 7.2 (equal at 256 tokens); softmax, whose scores need no work before they are ranked, 128
+// experts 2.6 / 2.1, 3.9 / 2.2, 9.2 / 2.7, 512 experts 9.1 / 6.9, 30.4 / 7.2, 102 / 9.3, 8 experts 1.7 / 1.5, 1.7 / 1.6, 3.0 / 1.8.
+static bool routes_by_counting(const RouteParams& p) {
+  if (p.num_expert_group > 1 && p.topk_group < p.num_expert_group) return p.n_tokens <= 1536;
+  return p.scoring == AKLR_SCORING_SIGMOID && static_cast<int64_t>(p.n_tokens) * p.n_routed <= 256 * 256;
+}
 
 static int check_route_shape(const RouteParams& p) {
   if (p.n_routed < 1 || p.n_routed > 1024 || p.topk < 1 || p.topk + p.n_shared > 32 || p.topk > p.n_routed)
@@ -346,7 +352,7 @@ static int check_route_shape(const RouteParams& p) {
 int launch_route(const RouteParams& p, cudaStream_t stream) {
   if (p.n_tokens == 0) return AKLR_OK;
   if (int rc = check_route_shape(p)) return rc;
-  if (p.n_tokens <= kCountingRouteTokens) {
+  if (routes_by_counting(p)) {
     const int per_token = p.n_routed < 32 ? 32 : (p.n_routed + 31) & ~31;
     return launch_kernel(route_count_kernel, dim3(p.n_tokens), dim3(per_token), 0, stream, 1, p) == cudaSuccess
                ? AKLR_OK : AKLR_ERR_CUDA;

@@ -113,3 +113,18 @@ def test_quantised_codes_do_not_depend_on_the_outputs_alignment(rows, hidden):
     assert torch.equal(codes.view(torch.uint8), codes8.view(torch.uint8)) and torch.equal(scales, scales8)
     amax = x.float().cpu().view(rows, hidden // 128, 128).abs().amax(-1)
     assert torch.equal(scales.cpu(), (amax.clamp_min(1e-10) * torch.tensor(1.0 / 448.0)).T.contiguous())
+
+
+@pytest.mark.parametrize("groups,limit", [(1, 256), (8, 1536)])
+def test_routing_is_the_same_on_both_sides_of_the_kernels_line(groups, limit):
+    """256 experts, sigmoid: counted up to 256 tokens without groups and 1536 with them, warp arg-maxes past that.  The
+    tables of the first tokens agree bit for bit."""
+    from aklr_b200.moe import Routing, route
+
+    g = torch.Generator().manual_seed(limit)
+    logits = torch.randn(limit + 1, 256, generator=g).to(torch.bfloat16).to(dev())
+    bias = (torch.randn(256, generator=g) * 0.01).to(dev())
+    routing = Routing(topk=8, scoring="sigmoid", num_expert_group=groups, topk_group=max(1, groups // 2), routed_scaling_factor=2.5)
+    ids, weights = route(logits, bias, routing)
+    ids_few, weights_few = route(logits[:limit].contiguous(), bias, routing)
+    assert torch.equal(ids[:limit], ids_few) and torch.equal(weights[:limit], weights_few)
