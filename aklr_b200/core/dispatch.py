@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import inspect
 import json
+import keyword
 import logging
 import os
 import threading
@@ -194,16 +195,25 @@ class CallRecorder:
 
 
 def _binder(signature: inspect.Signature, name: str) -> Callable[..., dict]:
-    """A function of exactly ``signature``'s parameters that returns them as a dict, defaults filled in.
+    """A function that binds a call's arguments as ``signature`` does and returns them as a dict, defaults filled in.
 
-    The interpreter binds a call's arguments to it in well under a microsecond; ``Signature.bind`` walks them in Python
-    and takes 5-10, which a decode call of a small layer waits for (its kernels are launched as fast as the host calls)."""
+    Where every parameter is an ordinary one, as in all of this package's ops, it is a generated function of exactly those
+    parameters: the interpreter binds a call to it in well under a microsecond; ``Signature.bind`` walks them in Python and
+    takes 5-10, which a decode call of a small layer waits for (its kernels are launched as fast as the host calls).  Any
+    other signature a contract is given (keyword-only parameters, a function without a plain name) binds by its own rules."""
+    ordinary = all(p.kind is p.POSITIONAL_OR_KEYWORD for p in signature.parameters.values())
+    if not (ordinary and name.isidentifier() and not keyword.iskeyword(name)):
+
+        def bind(*args, **kwargs):
+            bound = signature.bind(*args, **kwargs)
+            bound.apply_defaults()
+            return dict(bound.arguments)
+
+        return bind
     defaults = {f"_default_{p.name}": p.default for p in signature.parameters.values() if p.default is not p.empty}
-    parameters = []
-    for p in signature.parameters.values():
-        if p.kind is not p.POSITIONAL_OR_KEYWORD:
-            raise TypeError(f"{name}: parameter {p.name} must be an ordinary one")
-        parameters.append(p.name + (f"=_default_{p.name}" if p.default is not p.empty else ""))
+    parameters = [
+        p.name + (f"=_default_{p.name}" if p.default is not p.empty else "") for p in signature.parameters.values()
+    ]
     items = ", ".join(f"{p!r}: {p}" for p in signature.parameters)
     namespace = dict(defaults)
     exec(f"def {name}({', '.join(parameters)}):\n    return {{{items}}}", namespace)

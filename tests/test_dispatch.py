@@ -266,3 +266,29 @@ def test_api_arguments_bind_as_their_signature_does():
             signature.bind(*args, **kwargs)
         with pytest.raises(TypeError):
             bind(*args, **kwargs)
+
+
+def test_an_api_function_of_any_signature_is_accepted():
+    """Keyword-only parameters, and a function without a plain name, are declared and bound as ``inspect`` binds them."""
+    from aklr_b200.core.dispatch import KernelDispatcher, OpContract, Param
+
+    seen = []
+    contract = OpContract("probe@1", (Param("a"), Param("b", 2)), ("out",), key=lambda call: (1,),
+                          alloc=lambda call, key: None, run=lambda call, out: seen.append(dict(call)))
+
+    def keyword_only(a, *, b=2): ...
+
+    for fn in (keyword_only, lambda a, b=2: None):
+        dispatcher = KernelDispatcher(contract)
+        api_fn = dispatcher.make_api_fn(fn)
+        dispatcher.open()
+        seen.clear()
+        api_fn(1)
+        api_fn(a=1, b=3)
+        assert seen == [{"a": 1, "b": 2}, {"a": 1, "b": 3}]
+        with pytest.raises(TypeError):
+            api_fn()
+        with pytest.raises(TypeError):
+            api_fn(1, c=2)
+    with pytest.raises(TypeError):
+        KernelDispatcher(contract).make_api_fn(keyword_only)(1, 2)
