@@ -249,6 +249,7 @@ int check_config(const aklr_moe_config& c) {
 }
 
 int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
+bool is_aligned(const void* p, uintptr_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; }
 
 void layout_of(const aklr_moe_config& c, aklr_moe_workspace_layout* l) {
   const int64_t routes_per_token = c.topk + c.n_shared;
@@ -1220,6 +1221,8 @@ int64_t aklr_moe_align_max_blocks(int64_t n_routes, int64_t n_experts, int64_t b
 int aklr_router_gemm_bf16(const void* x, const void* w, void* logits, int32_t n_tokens, int32_t hidden,
                           int32_t n_routed, void* stream) {
   if (!x || !w || !logits) return fail(AKLR_ERR_BAD_ARGUMENT, "NULL argument");
+  if (!is_aligned(x, 16) || !is_aligned(w, 16) || !is_aligned(logits, 2))
+    return fail(AKLR_ERR_BAD_ARGUMENT, "router GEMM: x and w must be 16-byte aligned, logits 2-byte aligned");
   int rc = check_device();
   if (rc) return rc;
   // 64 tokens and up: tensor cores (128-token tiles); fewer: the warp-per-dot-product kernel, which
@@ -1302,11 +1305,13 @@ int aklr_tile_weights_fp8(const void* src, void* dst, int64_t matrices, int32_t 
 int aklr_router_gemm_f32(const void* x, const float* w, float* logits, int32_t n_tokens, int32_t hidden,
                          int32_t n_routed, void* stream) {
   if (!x || !w || !logits) return fail(AKLR_ERR_BAD_ARGUMENT, "NULL argument");
+  if (!is_aligned(x, 8) || !is_aligned(w, 16) || !is_aligned(logits, 4))
+    return fail(AKLR_ERR_BAD_ARGUMENT, "router GEMM (float32 weights): x must be 8-byte aligned, w 16-byte, logits 4-byte");
   int rc = check_device();
   if (rc) return rc;
-  // From 17 tokens on the tensor cores; below them, and for token rows that a TMA load cannot start at, dot products.
-  if (n_tokens > 16 && n_routed >= 1 && hidden % 128 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 &&
-      reinterpret_cast<uintptr_t>(w) % 16 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0) {
+  // From 17 tokens on the tensor cores; below them dot products.  The CUDA-core tile takes token rows that a TMA load
+  // cannot start at and logits that 16-byte stores cannot.
+  if (n_tokens > 16 && n_routed >= 1 && hidden % 128 == 0 && is_aligned(x, 16) && is_aligned(logits, 16)) {
     CUtensorMap map_x, map_w;
     rc = make_map_bf16(&map_x, x, n_tokens, hidden, 128);
     if (rc) return rc;

@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   } else {
     const int quarter = warp & 3;
     const int token = tok0 + quarter * 32 + lane;
+    const bool wide = (p.n_routed & 7) == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0;  // 16-byte stores start on their boundary
     const bool got = mbar_wait(acc_full, 0, abort_flag, status, 33);
     tc_fence_after_sync();
     const uint32_t t0 = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
       tc_wait_ld();
       if (got && token < p.n_tokens) {
         uint16_t* dst = p.logits + static_cast<size_t>(token) * p.n_routed + exp0 + c;
-        if (exp0 + c + 16 <= p.n_routed && (p.n_routed & 7) == 0) {
+        if (wide && exp0 + c + 16 <= p.n_routed) {
           uint32_t o[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {

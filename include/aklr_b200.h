@@ -322,12 +322,15 @@ int aklr_selftest_exact_divide(const float* x, const float* scale, int64_t n, in
 int aklr_tile_weights_fp8(const void* src, void* dst, int64_t matrices, int32_t rows, int32_t cols, void* stream);
 
 /* logits float32 [T,E] = x (bf16 [T,H]) @ w (float32 [E,H])^T, nothing rounded: the gate of
- * `minimax_m2_fp8_moe` (aklr/plugins/sglang/models/minimax_m2/reference.py:43-50). */
+ * `minimax_m2_fp8_moe` (aklr/plugins/sglang/models/minimax_m2/reference.py:43-50).  hidden a multiple of 128; x 8-byte,
+ * w 16-byte, logits 4-byte aligned, else AKLR_ERR_BAD_ARGUMENT (from 17 tokens on the tensor cores serve the call where
+ * x and logits are 16-byte aligned, a slower kernel where they are not). */
 int aklr_router_gemm_f32(const void* x, const float* w, float* logits, int32_t n_tokens, int32_t hidden,
                          int32_t n_routed, void* stream);
 
 /* logits bf16 [T,E] = bf16(x [T,H] @ w [E,H]^T): `_router_logits`
- * (aklr/plugins/sglang/models/qwen3_moe/reference.py:24-31). */
+ * (aklr/plugins/sglang/models/qwen3_moe/reference.py:24-31).  hidden a multiple of 8; x and w 16-byte, logits 2-byte
+ * aligned, else AKLR_ERR_BAD_ARGUMENT. */
 int aklr_router_gemm_bf16(const void* x, const void* w, void* logits, int32_t n_tokens, int32_t hidden,
                           int32_t n_routed, void* stream);
 

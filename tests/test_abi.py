@@ -99,3 +99,19 @@ def test_compute_calls_fail_loudly_without_a_device():
     x = torch.zeros((4, 128), dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="no CPU path"):
         moe.act_quant_fp8(x)
+
+
+@pytest.mark.parametrize("entry,x,w,logits", [
+    ("aklr_router_gemm_f32", 8, 8, 16),  # the weight is read 16 bytes at a time by every kernel
+    ("aklr_router_gemm_f32", 4, 16, 16),  # token rows 8 bytes at a time
+    ("aklr_router_gemm_f32", 16, 16, 2),
+    ("aklr_router_gemm_bf16", 8, 16, 16),  # both operands 16 bytes at a time, whatever the token count
+    ("aklr_router_gemm_bf16", 16, 8, 16),
+    ("aklr_router_gemm_bf16", 16, 16, 1),
+])
+@pytest.mark.parametrize("tokens", [1, 63, 64, 300])
+def test_router_operands_at_unreadable_addresses_are_refused(lib, entry, x, w, logits, tokens):
+    """Refused by the host, before anything looks at the memory: the addresses here are nobody's."""
+    base = 1 << 20
+    assert getattr(lib, entry)(base + x, base + w, base + logits, tokens, 256, 32, None) == -1
+    assert b"aligned" in lib.aklr_last_error()

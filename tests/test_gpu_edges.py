@@ -128,3 +128,19 @@ def test_routing_is_the_same_on_both_sides_of_the_kernels_line(groups, limit):
     ids, weights = route(logits, bias, routing)
     ids_few, weights_few = route(logits[:limit].contiguous(), bias, routing)
     assert torch.equal(ids[:limit], ids_few) and torch.equal(weights[:limit], weights_few)
+
+
+@pytest.mark.parametrize("tokens,experts", [(63, 64), (64, 64), (130, 256), (130, 33)])
+def test_bf16_router_writes_logits_of_any_address(tokens, experts):
+    """Logits that 16-byte stores cannot start at: bit for bit those of an aligned buffer, and nothing beside them."""
+    from aklr_b200 import _lib
+    from aklr_b200.moe import router_logits
+
+    x, w, _, _ = router_case(tokens, 256, experts, torch.bfloat16)
+    x, w = x.to(dev()), w.to(dev())
+    want = router_logits(x, w)
+    buffer = torch.full((tokens * experts + 16,), 7.0, dtype=torch.bfloat16, device=dev())
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.load().aklr_router_gemm_bf16(x.data_ptr(), w.data_ptr(), buffer.data_ptr() + 6, tokens, 256, experts, stream))
+    assert torch.equal(buffer[3 : 3 + tokens * experts].view(tokens, experts), want)
+    assert (buffer[:3] == 7.0).all() and (buffer[3 + tokens * experts :] == 7.0).all()
