@@ -178,7 +178,9 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
 // is the sum of three bf16 terms (its 24 significant bits cut into 8 + 8 + 8, exact short of underflow), a product of two
 // bf16 values is exact in float32, and the three products' sums are kept apart and added once, smallest first.  So the only roundings are those of the accumulation, 1/12th as many per element as a
 // CUDA-core chain over H has (K = 16 per MMA), in kF32Slices accumulators of the first term that share K out between them.
-// (An infinite activation meets zero low terms and makes its logits NaN; the quantiser makes that token NaN anyway.)
+// An infinite activation times a low term that is zero is NaN where the product itself is infinite, so a logit whose first
+// term is not finite is that term's sum alone: +-inf and NaN come out as from the CUDA-core kernels, whatever the batch
+// size.  (The first term of a weight below 2^-133 is zero too: its product with an infinity is NaN here.)
 //
 // One CTA per 128 tokens x 32 experts, 64 of K per stage: TMA loads the bf16 token tile (16 KB, SWIZZLE_128B) and the
 // raw weights (32 x 64 floats), four warps turn the weights into one 96-row operand tile (32 rows of each term, swizzled
@@ -351,6 +353,24 @@ __global__ void __launch_bounds__(kF32Threads, 1) router_gemm_f32_tc_kernel(cons
           tc_wait_ld();
 #pragma unroll
           for (int i = 0; i < 16; ++i) sum[i] += __uint_as_float(r[i]);
+        }
+        bool finite = true;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) finite = finite && isfinite(sum[i]);
+        if (!__all_sync(0xFFFFFFFFu, finite)) {  // see above: infinities meet the low terms' zeros
+          float first[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) first[i] = 0.0f;
+          for (int sl = 0; sl < slices; ++sl) {
+            uint32_t r[16];
+            AKLR_TMEM_LD_16(t0 + (2 + sl) * kF32Experts + c, r);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) first[i] += __uint_as_float(r[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (!isfinite(first[i])) sum[i] = first[i];
         }
         if (token < p.n_tokens) {
           float* dst = p.logits + static_cast<size_t>(token) * p.n_routed + exp0 + c;

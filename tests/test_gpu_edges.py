@@ -55,6 +55,34 @@ def test_float32_router_keeps_float32_accuracy(tokens, hidden, experts):
         assert ((again - exact).abs() <= (hidden + 32) * 2.0**-24 * magnitude).all()
 
 
+@pytest.mark.parametrize("tokens", [1, 16, 17, 130])
+@pytest.mark.parametrize("experts", [33, 256])
+def test_router_infinities_do_not_depend_on_the_batch_size(tokens, experts):
+    """An infinite activation or weight gives +-inf, NaN where it meets a zero or the opposite infinity, and a NaN gives
+    NaN, from the dot products (up to 16 tokens) and from the tensor cores alike; all other logits are as without them."""
+    from aklr_b200.moe import router_logits, router_logits_f32
+
+    g = torch.Generator().manual_seed(tokens + experts)
+    x = torch.randn(tokens, 384, generator=g).to(torch.bfloat16)
+    w = (torch.randn(experts, 384, generator=g) * 0.05).to(torch.bfloat16).float()
+    w[7, 100] = 0.0
+    w[9, 200], w[10, 300], w[11, 44] = float("inf"), float("-inf"), float("nan")
+    x[0, 100] = float("inf")
+    if tokens > 1:
+        x[1, 5], x[2, 5], x[2, 333] = float("-inf"), float("inf"), float("inf")
+        x[3, 17], x[tokens - 1, 200] = float("nan"), float("-inf")
+    products = x.double()[:, None, :] * w.double()[None]
+    exact = products.sum(-1)
+    finite = exact.isfinite()
+    assert exact.isposinf().any() and exact.isneginf().any() and exact.isnan().any()
+    bound = (384 / 16 + 32) * 2.0**-23 * products.abs().nan_to_num(0.0, 0.0, 0.0).sum(-1)
+    for weight, logits, rounding in ((w, router_logits_f32, 0.0), (w.to(torch.bfloat16), router_logits, 2.0**-8)):
+        got = logits(x.to(dev()), weight.to(dev())).cpu().double()
+        assert torch.equal(got.isnan(), exact.isnan())
+        assert torch.equal(got.isposinf(), exact.isposinf()) and torch.equal(got.isneginf(), exact.isneginf())
+        assert ((got - exact).abs()[finite] <= (rounding * exact.abs() + bound)[finite]).all()
+
+
 @pytest.mark.parametrize("n_experts", [1, 31, 543, 544, 545, 1025])
 @pytest.mark.parametrize("n_tokens,k,block_m", [(1, 1, 16), (33, 1, 128), (1025, 1, 16), (4096, 1, 32), (4097, 1, 128)])
 def test_sort_with_and_without_the_per_warp_counts(n_experts, n_tokens, k, block_m):
