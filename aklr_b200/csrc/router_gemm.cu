@@ -1,7 +1,7 @@
 // Router projection on the tensor cores, sm_100a: logits[T, E] = bf16( x[T, H] . W[E, H]^T ) with
 // float32 accumulation in TMEM, the rounding point of the reference's _router_logits
 // (aklr/plugins/sglang/models/qwen3_moe/reference.py:24-31).  One CTA per 128 tokens x 16..256
-// experts: TMA (SWIZZLE_128B, 64 bf16 = 128 bytes of K per box, two boxes per stage) feeds
+// experts: TMA (SWIZZLE_128B, 64 bf16 = 128 bytes of K per box, one or two boxes per stage) feeds
 // tcgen05.mma kind::f16 (M128, N = experts of the tile, K16); rows and experts past the end are zero-filled by the
 // TMA.  192 threads: warp 0 TMA, warp 1 MMA + TMEM, warps 2..5 epilogue (one TMEM lane quarter each).
 //
@@ -29,7 +29,6 @@ struct RouterParams {
   int32_t* status;    // optional [2]
   int32_t* host_status;  // the device's host-visible copy of a failure (or null)
   int n_tokens, hidden, n_routed, n_tile, stages;
-  int boxes;  // 64-wide boxes of K per stage: 2 where hidden allows
 };
 
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
@@ -42,10 +41,17 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
       : "memory");
 }
 
+// BOXES: 64-wide boxes of K per stage, two where hidden allows and the tile leaves room for three such stages and more
+// (256 experts do not: two of 96 KB, at which 16384 tokens on 7168 x 256 took 69-71 us, 62-65 with four stages of one box).
+// LONE_LANE: one lane of the producer and of the MMA warp waits and issues, the others stand by, in place of the whole warp
+// waiting and an elected lane issuing.  Cheap issue does not matter where an MMA of 256 columns outlasts it, and the vote
+// after every wait then is one hand-off more in a ring of four stages: 9600 / 16384 / 32768 tokens on 7168 x 256 51 / 62 /
+// 121 us by the warp, 48 / 58 / 115 by the lane; below 256 columns the lane is the slower (300 tokens: 19 / 27).
+template <int BOXES, bool LONE_LANE>
 __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __grid_constant__ RouterParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int box_bytes = kABytes + p.n_tile * 128, stage_bytes = p.boxes * box_bytes;
+  const int box_bytes = kABytes + p.n_tile * 128, stage_bytes = BOXES * box_bytes;
   const int kStages = p.stages;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * stage_bytes);
   uint64_t* empty = full + kStages;
@@ -59,7 +65,7 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   int* status = p.status ? p.status : local_status;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k_steps = (p.hidden >> 6) / p.boxes;
+  const int k_steps = (p.hidden >> 6) / BOXES;
   const int tok0 = blockIdx.x * 128, exp0 = blockIdx.y * p.n_tile;
   uint32_t tmem_cols = 32;
   while (tmem_cols < static_cast<uint32_t>(p.n_tile)) tmem_cols <<= 1;
@@ -86,36 +92,42 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
   const uint32_t tmem_base = *tmem_ptr;
   griddep_wait();
   griddep_launch();
+  auto wait = [&](uint64_t* bar, uint32_t parity, int where) {
+    return LONE_LANE ? mbar_wait(bar, parity, abort_flag, status, where) : mbar_wait_warp(bar, parity, abort_flag, status, where);
+  };
+  const bool stands_by = LONE_LANE && warp < 2 && lane != 0;
 
   if (warp == 0) {
-    const bool leader = elect_one();
+    const bool leader = LONE_LANE || elect_one();
     int s = 0;
     uint32_t ph = 0;
-    for (int it = 0; it < k_steps; ++it) {
-      if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, status, 31)) break;
+    for (int it = stands_by ? k_steps : 0; it < k_steps; ++it) {
+      if (!wait(&empty[s], ph ^ 1, 31)) break;
       uint8_t* st = smem + s * stage_bytes;
       if (leader) {
         mbar_expect_tx(&full[s], stage_bytes);
-        for (int b = 0; b < p.boxes; ++b) {
-          tma_load_2d(st + b * box_bytes, &p.map_x, &full[s], (it * p.boxes + b) * 64, tok0);
-          tma_load_2d(st + b * box_bytes + kABytes, &p.map_w, &full[s], (it * p.boxes + b) * 64, exp0);
+#pragma unroll
+        for (int b = 0; b < BOXES; ++b) {
+          tma_load_2d(st + b * box_bytes, &p.map_x, &full[s], (it * BOXES + b) * 64, tok0);
+          tma_load_2d(st + b * box_bytes + kABytes, &p.map_w, &full[s], (it * BOXES + b) * 64, exp0);
         }
       }
       if (++s == kStages) { s = 0; ph ^= 1; }
     }
   } else if (warp == 1) {
-    const bool leader = elect_one();
+    const bool leader = LONE_LANE || elect_one();
     // kind::f16: f32 accumulator, bf16 A and B, K-major, M 128, N n_tile
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(p.n_tile >> 3) << 17) |
                            (static_cast<uint32_t>(128 >> 4) << 24);
-    bool ok = true;
+    bool ok = !stands_by;
     int s = 0;
     uint32_t ph = 0;
-    for (int it = 0; it < k_steps; ++it) {
-      if (!mbar_wait_warp(&full[s], ph, abort_flag, status, 32)) { ok = false; break; }
+    for (int it = 0; it < k_steps && ok; ++it) {
+      if (!wait(&full[s], ph, 32)) { ok = false; break; }
       tc_fence_after_sync();
       if (leader) {
-        for (int b = 0; b < p.boxes; ++b) {
+#pragma unroll
+        for (int b = 0; b < BOXES; ++b) {
           const uint32_t a0 = smem_u32(smem + s * stage_bytes + b * box_bytes);
           const uint64_t da = umma_desc_sw128(a0), db = umma_desc_sw128(a0 + kABytes);
 #pragma unroll
@@ -423,14 +435,15 @@ int launch_router_gemm_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, vo
   p.hidden = hidden;
   p.n_routed = n_routed;
   p.n_tile = n_tile;
-  p.boxes = hidden % 128 == 0 ? 2 : 1;
-  const int stage_bytes = p.boxes * (kABytes + n_tile * 128);
+  const int boxes = hidden % 128 == 0 && n_tile < 256 ? 2 : 1;
+  const int stage_bytes = boxes * (kABytes + n_tile * 128);
   p.stages = kSmemBudget / stage_bytes;
   if (p.stages > kMaxStages) p.stages = kMaxStages;
   const size_t smem = static_cast<size_t>(p.stages) * stage_bytes + (2 * p.stages + 1) * 8 + 32 + 1024;
-  if (ensure_max_dynamic_smem(reinterpret_cast<const void*>(router_gemm_tc_kernel)) != AKLR_OK) return AKLR_ERR_CUDA;
+  auto* kernel = n_tile == 256 ? router_gemm_tc_kernel<1, true> : boxes == 2 ? router_gemm_tc_kernel<2, false> : router_gemm_tc_kernel<1, false>;
+  if (ensure_max_dynamic_smem(reinterpret_cast<const void*>(kernel)) != AKLR_OK) return AKLR_ERR_CUDA;
   const dim3 grid((n_tokens + 127) / 128, (n_routed + n_tile - 1) / n_tile);
-  return launch_kernel(router_gemm_tc_kernel, grid, dim3(kThreads), smem, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  return launch_kernel(kernel, grid, dim3(kThreads), smem, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 int launch_router_gemm_f32_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, float* logits, int n_tokens, int hidden,

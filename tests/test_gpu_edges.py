@@ -37,6 +37,33 @@ def test_bf16_router_at_every_shape_of_its_kernels(tokens, hidden, experts):
     assert ((got - exact).abs() <= 2.0**-8 * exact.abs() + (hidden / 16 + 16) * 2.0**-23 * magnitude).all()
 
 
+def router_tile(tokens, experts, sms):
+    """Experts per CTA of the bf16 tensor-core router: the fewest, a power of two from 16, whose CTAs fit the chip at once."""
+    tile = 16
+    while tile < 256 and tile < experts and -(-tokens // 128) * -(-experts // tile) > sms:
+        tile *= 2
+    return tile
+
+
+@pytest.mark.parametrize("hidden", [192, 256])
+@pytest.mark.parametrize("tokens,experts,tile", [(1153, 256, 32), (3999, 250, 64), (4097, 257, 128), (9601, 257, 256), (16385, 256, 256)])
+def test_bf16_router_at_every_width_of_its_tiles(hidden, tokens, experts, tile):
+    """Tiles of 32 to 256 experts, ragged in experts and in tokens: the bound of the test above, and bit for bit the logits
+    that the same rows get from calls small enough for 16-expert tiles (one accumulation over K whatever the tile)."""
+    from aklr_b200.moe import router_logits
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert router_tile(tokens, experts, sms) == tile
+    x, w, exact, magnitude = router_case(tokens, hidden, experts, torch.bfloat16)
+    x, w = x.to(dev()), w.to(dev())
+    got = router_logits(x, w)
+    error = (got.cpu().double() - exact).abs()
+    assert (error <= 2.0**-8 * exact.abs() + (hidden / 16 + 16) * 2.0**-23 * magnitude).all()
+    for rows in (slice(0, 512), slice(tokens - 129, tokens)):
+        assert router_tile(x[rows].shape[0], experts, sms) == 16
+        assert torch.equal(got[rows], router_logits(x[rows].contiguous(), w))
+
+
 @pytest.mark.parametrize("tokens", [1, 16, 17, 128, 129, 300])
 @pytest.mark.parametrize("hidden,experts", [(128, 1), (384, 33), (768, 40), (3072, 256)])
 def test_float32_router_keeps_float32_accuracy(tokens, hidden, experts):
