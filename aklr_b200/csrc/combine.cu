@@ -283,10 +283,10 @@ int launch_add_gated_rows(const void* x, const void* gate, const void* rows, voi
 //  * few tokens: one warp per (token, expert) dot product, so the weight is read by many SMs;
 //  * else the tensor cores (router_gemm.cu); this file keeps a 64 x 64 tile per CTA, 16 k per step, 4 x 4 outputs per
 //    thread, for token rows a TMA load cannot start at.
+template <int UNROLL>  // strides whose loads are in flight together (see router_gemm_kernel)
 __global__ void __launch_bounds__(256)
 router_dot_f32_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,
                       int n_tokens, int hidden, int n_routed) {
-  constexpr int UNROLL = 8;  // strides whose loads are in flight together (see router_gemm_kernel)
   const int lane = threadIdx.x & 31;
   const int64_t item = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   griddep_wait();
@@ -374,7 +374,9 @@ int launch_router_gemm_f32(const void* x, const float* w, float* logits, int n_t
   auto* xp = static_cast<const uint16_t*>(x);
   if (n_tokens <= 16) {
     const int64_t blocks = (static_cast<int64_t>(n_tokens) * n_routed + 7) / 8;
-    return launch_kernel(router_dot_f32_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, 1, xp, w, logits, n_tokens,
+    // Eight strides in flight take 66 registers a thread, three CTAs per SM: from 512 CTAs on, more CTAs with four strides hide
+    // as much (eight / four: 12 tokens on 7168 x 384 12.4 / 10.0 us, 16 on 3072 x 256 6.4 / 4.9; 8 on 7168 x 384 8.0 / 9.3).
+    return launch_kernel(blocks < 512 ? router_dot_f32_kernel<8> : router_dot_f32_kernel<4>, dim3(static_cast<unsigned>(blocks)), dim3(256), 0, stream, 1, xp, w, logits, n_tokens,
                          hidden, n_routed) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
   }
   const dim3 grid((n_tokens + 63) / 64, (n_routed + 63) / 64);
