@@ -1,6 +1,6 @@
-// Per-token-group FP8 activation quantisation, sm_100a.  All three kernels are HBM-bound
-// element-wise passes: 16-byte loads (8 bf16 per lane), shuffle reductions inside the lanes of
-// one group, 8-byte stores.
+// Per-token-group FP8 activation quantisation, sm_100a: element-wise passes on 16-byte loads with shuffle reductions
+// inside the lanes of one group.  The two 1 x 128 kernels hold 16 or 8 values per lane (quant_rows.cuh says when) and
+// store them in one 16-byte or 8-byte word; the 1 x 32 kernel holds 8.
 //
 //  * gather_quant_fp8: the MoE layer's scheme -- scale = max(amax/448, FLT_MIN), code =
 //    e4m3(x / scale), both true divisions, as the reference's _fp8_input does
@@ -18,11 +18,12 @@
 
 namespace aklr {
 
+template <int LANES>
 __global__ void __launch_bounds__(256) gather_quant_fp8_kernel(GatherQuantParams p) {
   griddep_wait();
   griddep_launch();
-  gather_quant_fp8_groups(p, (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kGroupLanes,
-                          (static_cast<int64_t>(gridDim.x) * blockDim.x) / kGroupLanes);
+  gather_quant_fp8_groups<LANES>(p, (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / LANES,
+                                 (static_cast<int64_t>(gridDim.x) * blockDim.x) / LANES);
 }
 
 // Rows already quantised elsewhere (each token once, or by the sender of an expert-parallel
@@ -87,28 +88,36 @@ int launch_gather_quant_fp8(const GatherQuantParams& p, cudaStream_t stream) {
   if (p.n_rows == 0) return AKLR_OK;
   const int64_t groups = static_cast<int64_t>(p.n_rows) * (p.hidden / 128);
   if (groups >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
-  const int64_t blocks = (groups * kGroupLanes + 255) / 256;
+  // A layer's gather (num_rows set) launches for the table's capacity, and twice the CTAs for rows that are not there cost
+  // more than the shorter chain gains: 17 tokens x 11 routes on 2048 x 128, 55.3 us for the call with 8 lanes, 56.0 with 16.
+  const int lanes = p.num_rows ? 8 : quant_lanes(groups);
+  const int64_t blocks = (groups * lanes + 255) / 256;
   const int grid = static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16);
-  return launch_kernel(gather_quant_fp8_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  return launch_kernel(lanes == 16 ? gather_quant_fp8_kernel<16> : gather_quant_fp8_kernel<8>, dim3(grid), dim3(256), 0, stream, 1, p) ==
+                 cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
+template <int LANES>
 __global__ void __launch_bounds__(256)
 per_group_quant_fp8_kernel(const uint16_t* __restrict__ x, uint8_t* __restrict__ q,
                            float* __restrict__ scales, int rows, int hidden) {
+  using Values = GroupValues<LANES>;
   const int groups_per_row = hidden >> 7;
   const int64_t total = static_cast<int64_t>(rows) * groups_per_row;
-  const int sub = threadIdx.x & (kGroupLanes - 1);
-  const uint32_t group_mask = 0xFFu << (threadIdx.x & 24);
+  const int sub = Values::sub();
+  const uint32_t group_mask = Values::mask();
   const bool wide = reinterpret_cast<uintptr_t>(q) % 16 == 0;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x / kGroupLanes;
-  for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kGroupLanes; g < total; g += stride) {
-    GroupValues val;
-    val.load(x + g * 128 + sub * 16);  // groups of a row follow one another
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x / LANES;
+  for (int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / LANES; g < total; g += stride) {
+    Values val;
+    val.load(x + g * 128 + sub * Values::N);  // groups of a row follow one another
     const float scale = __fmul_rn(fmaxf(val.group_amax(group_mask), 1e-10f), 1.0f / 448.0f);
     const float recip = __fdiv_rn(1.0f, scale);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) val.v[i] = fminf(fmaxf(__fmul_rn(val.v[i], recip), -448.0f), 448.0f);
-    GroupValues::store(q + g * 128 + sub * 16, val.pack(), wide);
+    for (int i = 0; i < Values::N; ++i) val.v[i] = fminf(fmaxf(__fmul_rn(val.v[i], recip), -448.0f), 448.0f);
+    uint32_t codes[Values::N / 4];
+    val.pack(codes);
+    Values::store(q + g * 128 + sub * Values::N, codes, wide);
     if (sub == 0) {
       const uint32_t row = static_cast<uint32_t>(g) / static_cast<uint32_t>(groups_per_row);  // g < 2^31: checked at launch
       const uint32_t grp = static_cast<uint32_t>(g) - row * static_cast<uint32_t>(groups_per_row);
@@ -123,9 +132,11 @@ int launch_per_group_quant_fp8(const void* x, uint8_t* q, float* scales, int row
   if (rows == 0) return AKLR_OK;
   const int64_t groups = static_cast<int64_t>(rows) * (hidden / 128);
   if (groups >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
-  const int64_t blocks = (groups * kGroupLanes + 255) / 256;
+  const int lanes = quant_lanes(groups);
+  const int64_t blocks = (groups * lanes + 255) / 256;
   const int grid = static_cast<int>(blocks < 148 * 16 ? blocks : 148 * 16);
-  per_group_quant_fp8_kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(x), q, scales, rows, hidden);
+  auto* kernel = lanes == 16 ? per_group_quant_fp8_kernel<16> : per_group_quant_fp8_kernel<8>;
+  kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(x), q, scales, rows, hidden);
   return cudaGetLastError() == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
