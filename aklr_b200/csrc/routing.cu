@@ -429,17 +429,25 @@ __device__ int block_exclusive_scan(int v, int* scratch, int* total) {
   return inc - v + (warp > 0 ? scratch[warp - 1] : 0);
 }
 
-// -1 in the padding rows: from this block size on a warp per expert writes them (one thread per expert stores up to 127 of
-// them one after the other: 64 tokens on 257 experts in 128-row blocks, 21 -> 9 us for the sort with place_chunk's table).
-// Below it the thread that plans an expert does: 15 or 31 stores at most, and a decode call finds the code in its caches
-// (one token: 84.9 us for the call, 86.7 with the warps).
+// -1 in the padding rows: in blocks from kWarpFillBlock rows on a warp per expert writes them (one thread per expert stores
+// up to 127 of them one after the other: 64 tokens on 257 experts in 128-row blocks, 21 -> 8 us for the sort with
+// place_chunk's table).  Below it the thread that plans an expert does: 15 or 31 stores at most, and a decode call finds the
+// code in its caches (one token: 84.9 us for the call, 86.7 with the warps).  So it does where the routes are few for the
+// experts: the warps look at every expert, and most have no row.  128-row blocks, microseconds by threads / by warps: 1024
+// experts 8, 64, 128 routes 4.4 / 10.1, 8.5 / 11.0, 12.2 / 11.6; 513 experts 11, 44, 88 routes 4.8 / 6.8, 6.7 / 7.6, 9.2 / 8.2;
+// 257 experts 18, 36, 72 routes 4.6 / 5.4, 5.6 / 5.7, 7.8 / 6.2; 128 experts 16, 32 routes 4.2 / 4.5, 5.7 / 4.8; 8 experts,
+// which have a warp each, 3.8 / 3.4 for 2 routes.
 constexpr int kWarpFillBlock = 64;
+__device__ __forceinline__ bool threads_fill(const AlignParams& p) {
+  return p.block_m < kWarpFillBlock || (p.n_experts > 32 && p.n_routes <= 16 + p.n_experts / 13);
+}
 
 // Shared by the scan kernel and the one-CTA path: from per-expert totals in smem ``total`` compute
 // padded bases, the block table, counts, the pad fill.  ``base`` receives each expert's first row.
 __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, int* scratch) {
   // serial-in-chunks exclusive scan over experts of padded block counts (n_experts <= 1025)
   const int tid = threadIdx.x, nt = blockDim.x;
+  const bool by_threads = threads_fill(p);
   const int per = (p.n_experts + nt - 1) / nt;
   int local_sum = 0;
   for (int i = 0; i < per; ++i) {
@@ -479,13 +487,13 @@ __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, i
         for (int b = 0; b < nb; b += 2)
           p.pair_table[pair_running++] = (running + b) | (b + 1 < nb ? static_cast<int>(0x80000000u) : 0);
       }
-      if (p.block_m < kWarpFillBlock)
+      if (by_threads)
         for (int r = c; r < nb * p.block_m; ++r) p.sorted_ids[running * p.block_m + r] = -1;
       running += nb;
     }
   }
   __syncthreads();
-  if (p.block_m < kWarpFillBlock) return;
+  if (by_threads) return;
   for (int e = tid >> 5; e < p.n_experts; e += nt >> 5) {
     const int c = total[e], end = (c + p.block_m - 1) / p.block_m * p.block_m;
     for (int r = c + (tid & 31); r < end; r += 32) p.sorted_ids[base[e] + r] = -1;
