@@ -321,6 +321,13 @@ bool fused_prologue_serves(const aklr_moe_config& c) {
              aklr::kDecodePrologueExperts;
 }
 
+// A call refused after its workspace was accepted has no sort, which is what clears the status words: they are cleared
+// here, so that reading them finds neither an earlier call's failure nor what the memory held.
+int refused(int rc, const aklr_moe_workspace_layout& l, void* workspace, cudaStream_t stream) {
+  cudaMemsetAsync(static_cast<uint8_t*>(workspace) + l.status, 0, 8, stream);
+  return rc;
+}
+
 int run_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l, const void* hidden_states,
                 const int32_t* topk_ids, const float* topk_weights, const int32_t* expert_map,
                 int n_experts_global, const void* w1, const float* w1_scale, const void* w2,
@@ -362,11 +369,11 @@ int run_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l, co
   int rc = AKLR_OK;
   if (route) {
     rc = launch_decode_prologue(*route, ap, stream);
-    if (rc) return fail(rc, "decode prologue launch failed");
+    if (rc) return refused(fail(rc, "decode prologue launch failed"), l, ws, stream);
     g_launches += 1;
   } else {
     rc = launch_align(ap, stream);
-    if (rc) return fail(rc, "moe_align launch failed");
+    if (rc) return refused(fail(rc, "moe_align launch failed"), l, ws, stream);
     g_launches += routes <= 4096 ? 1 : 3;
   }
   profile_mark(stream, slot, 2);
@@ -510,7 +517,9 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
                    const uint8_t* q_in = nullptr, const uint8_t* scales_in = nullptr, void* rows_out = nullptr,
                    int slot = -1, int q_in_stride = 0, int scales_in_stride = 0) {
   using namespace aklr;
-  if (tiled_weights(c)) return fail(AKLR_ERR_BAD_ARGUMENT, "the tile-contiguous weight layout is an FP8 layout: packed MXFP4 weights stay row-major");
+  if (tiled_weights(c))
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "the tile-contiguous weight layout is an FP8 layout: packed MXFP4 weights stay row-major"),
+                   l, ws, stream);
   const int routes_per_token = c.topk + c.n_shared;
   const int routes = c.n_tokens * routes_per_token;
   const int experts = c.n_routed + c.n_shared;
@@ -535,7 +544,7 @@ int run_mx_experts(const aklr_moe_config& c, const aklr_moe_workspace_layout& l,
   ap.num_local_tokens = opt.num_local_tokens;
   ap.routes_per_token = routes_per_token;
   int rc = launch_align(ap, stream);
-  if (rc) return fail(rc, "moe_align launch failed");
+  if (rc) return refused(fail(rc, "moe_align launch failed"), l, ws, stream);
   g_launches += routes <= 4096 ? 1 : 3;
   profile_mark(stream, slot, 2);
 
@@ -808,7 +817,7 @@ int aklr_moe_fp8_forward(const aklr_moe_config* cfg, const void* hidden_states, 
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;  // nothing to do; empty tensors may have NULL pointers
   if (!hidden_states || !logits || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int32_t* ids = reinterpret_cast<int32_t*>(ws + l.topk_ids);
   float* weights = reinterpret_cast<float*>(ws + l.topk_weights);
@@ -821,7 +830,7 @@ int aklr_moe_fp8_forward(const aklr_moe_config* cfg, const void* hidden_states, 
                        w2_scale, out, ws, stream, slot, nullptr, nullptr, nullptr, &route);
   }
   rc = aklr_moe_route(cfg, logits, bias, sigmoid_table, ids, weights, stream_);
-  if (rc) return rc;
+  if (rc) return refused(rc, l, workspace, stream);
   profile_mark(stream, slot, 1);
   return run_experts(*cfg, l, hidden_states, ids, weights, nullptr, cfg->n_routed + cfg->n_shared, w1, w1_scale, w2,
                      w2_scale, out, ws, stream, slot);
@@ -837,10 +846,11 @@ int aklr_moe_fp8_experts(const aklr_moe_config* cfg, const void* hidden_states, 
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!hidden_states || !topk_ids || !topk_weights || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   const int local = cfg->n_routed + cfg->n_shared;
   const int global = expert_map ? cfg->n_experts_global : local;
-  if (expert_map && global < 1) return fail(AKLR_ERR_BAD_ARGUMENT, "n_experts_global must be set with an expert map");
+  if (expert_map && global < 1)
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "n_experts_global must be set with an expert map"), l, workspace, stream);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   profile_mark(stream, slot, 1);
@@ -859,7 +869,7 @@ int aklr_moe_fp8_experts_prequant(const aklr_moe_config* cfg, const void* rows_q
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!rows_q || !rows_scale || !expert_ids || !weights || !w1 || !w1_scale || !w2 || !w2_scale || !out_rows)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   profile_mark(stream, slot, 1);
@@ -886,10 +896,11 @@ int aklr_moe_mxfp4_experts_ex(const aklr_moe_config* cfg, const void* hidden_sta
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!hidden_states || !topk_ids || !topk_weights || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   const int local = cfg->n_routed + cfg->n_shared;
   const int global = expert_map ? cfg->n_experts_global : local;
-  if (expert_map && global < 1) return fail(AKLR_ERR_BAD_ARGUMENT, "n_experts_global must be set with an expert map");
+  if (expert_map && global < 1)
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "n_experts_global must be set with an expert map"), l, workspace, stream);
   return run_mx_experts(*cfg, l, hidden_states, topk_ids, topk_weights, expert_map, global, w1, w1_scale, w2, w2_scale,
                         *options, out, static_cast<uint8_t*>(workspace), stream);
 }
@@ -916,14 +927,14 @@ int aklr_moe_mxfp4_forward(const aklr_moe_config* cfg, const void* hidden_states
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!hidden_states || !logits || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   int32_t* ids = reinterpret_cast<int32_t*>(ws + l.topk_ids);
   float* weights = reinterpret_cast<float*>(ws + l.topk_weights);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   rc = aklr_moe_route(cfg, logits, bias, sigmoid_table, ids, weights, stream_);
-  if (rc) return rc;
+  if (rc) return refused(rc, l, workspace, stream);
   profile_mark(stream, slot, 1);
   return run_mx_experts(*cfg, l, hidden_states, ids, weights, nullptr, cfg->n_routed + cfg->n_shared, w1, w1_scale, w2,
                         w2_scale, clamp_only(swiglu_limit), out, ws, stream, nullptr, nullptr, nullptr, slot);
@@ -944,7 +955,7 @@ int aklr_moe_mxfp4_experts_prequant(const aklr_moe_config* cfg, const void* rows
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!rows_q || !rows_scale || !expert_ids || !weights || !w1 || !w1_scale || !w2 || !w2_scale || !out_rows)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   profile_mark(stream, slot, 1);
@@ -966,9 +977,9 @@ int aklr_moe_fp8_experts_rows(const aklr_moe_config* cfg, const void* rows_q, in
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!rows_q || !rows_scale || !topk_ids || !topk_weights || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   if (reinterpret_cast<uintptr_t>(rows_q) % 16 != 0 || reinterpret_cast<uintptr_t>(rows_scale) % 4 != 0)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "rows_q must be 16-byte aligned and rows_scale 4-byte aligned");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "rows_q must be 16-byte aligned and rows_scale 4-byte aligned"), l, workspace, stream);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   profile_mark(stream, slot, 1);
@@ -993,9 +1004,9 @@ int aklr_moe_mxfp4_experts_rows(const aklr_moe_config* cfg, const void* rows_q, 
   if (rc) return rc;
   if (cfg->n_tokens == 0) return AKLR_OK;
   if (!rows_q || !rows_scale || !topk_ids || !topk_weights || !w1 || !w1_scale || !w2 || !w2_scale || !out)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "NULL tensor argument"), l, workspace, stream);
   if (reinterpret_cast<uintptr_t>(rows_q) % 16 != 0 || reinterpret_cast<uintptr_t>(rows_scale) % 4 != 0)
-    return fail(AKLR_ERR_BAD_ARGUMENT, "rows_q must be 16-byte aligned and rows_scale 4-byte aligned");
+    return refused(fail(AKLR_ERR_BAD_ARGUMENT, "rows_q must be 16-byte aligned and rows_scale 4-byte aligned"), l, workspace, stream);
   const int slot = profile_slot();
   profile_mark(stream, slot, 0);
   profile_mark(stream, slot, 1);

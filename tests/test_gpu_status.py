@@ -64,3 +64,34 @@ def test_selftest_rejects_limits_that_could_stall_a_device():
     assert lib.aklr_selftest_wait_expiry(0, status.data_ptr(), None) == -1
     assert lib.aklr_selftest_wait_expiry(5_000_000_000, status.data_ptr(), None) == -1
     assert lib.aklr_selftest_wait_expiry(1000, None, None) == -1
+
+
+@pytest.mark.parametrize("entry", ["aklr_moe_fp8_experts", "aklr_moe_fp8_forward", "aklr_moe_mxfp4_experts", "aklr_moe_mxfp4_forward"])
+@pytest.mark.parametrize("refusal", ["tensor", "routing", "layout"])
+def test_a_refused_call_leaves_clear_status_words(entry, refusal):
+    """A workspace of whatever the memory held, a call that its arguments rule out before anything is launched: no failure
+    is read from the workspace afterwards, as after a call that was served."""
+    from aklr_b200 import _lib
+    from aklr_b200.moe import Routing, Workspace, _config
+
+    if (refusal == "routing" and "forward" not in entry) or (refusal == "layout" and "mxfp4" not in entry):
+        pytest.skip("only calls that route refuse a routing, only MXFP4 weights a tiled layout")
+    lib = _lib.load()
+    mx = "mxfp4" in entry
+    cfg = _config(4, 256, 128, 8, Routing(topk=2, scoring="sigmoid"), block_m=128 if mx else 16)
+    if refusal == "routing":
+        cfg.num_expert_group, cfg.topk_group = 3, 1  # eight experts do not make three groups
+    if refusal == "layout":
+        cfg.variant |= _lib.VARIANT_TILED_WEIGHTS
+    ws = Workspace(cfg, torch.device("cuda:0"))
+    ws.buffer.fill_(0xFF)
+    stream = torch.cuda.current_stream().cuda_stream
+    some = ws.base_ptr  # stands for the tensors: at most the routing is launched, which reads 64 bytes of logits
+    first = None if refusal == "tensor" else some
+    head = (ctypes.byref(cfg), first, some, some, None) if "experts" in entry else (ctypes.byref(cfg), first, some, None, None)
+    clamp = (0.0,) if mx else ()
+    before = lib.aklr_kernel_launch_count()
+    assert getattr(lib, entry)(*head, some, some, some, some, *clamp, some, ws.base_ptr, ws.layout.total_bytes, stream) != 0
+    if refusal != "layout" or "forward" not in entry:  # (the layout is looked at after the routing)
+        assert lib.aklr_kernel_launch_count() == before
+    ws.check_status()
