@@ -378,7 +378,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
 #pragma unroll
       for (int d = 0; d < kDepth; ++d) {
         if (it0 + 2 * d < total_its && ok) {
-          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status, 25)) ok = false;
+          // one verdict for the warp: a lane that gave up alone would leave the others at the __syncwarp below for good
+          ok = mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, p.status, 25);
           uint8_t* sf = smem + s * kStageBytes + kOffSf;
           *reinterpret_cast<uint4*>(sf + lane * 16) = aq[d];
           if (SPLIT) *reinterpret_cast<uint4*>(sf + kSfLoOffset + lane * 16) = aq_lo[SPLIT ? d : 0];
