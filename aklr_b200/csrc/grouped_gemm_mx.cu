@@ -626,38 +626,40 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_mx_kernel(const __gr
 }
 
 // Four lanes x 8 values per 1 x 32 group: rows gathered through the sorted route table, e4m3 codes row-major, scale
-// bytes in tcgen05.cp order.  A CTA column works on one 128-row block: its routed rows come first, so their count -- one
-// look at the block's ids -- is all the work there is, plus zero codes for the padding rows that the GEMM's producer
-// loads.  A warp takes 1024 values of a row at a time, all four 16-byte loads of a lane in flight.  (Walking every row
-// of the table, padding included, took 65 us for 64 tokens on 231 experts, of which 576 rows of 29.6 k are routed.)
-constexpr int kMxQuantSegment = 1024;  // values of a row per warp and pass
-__global__ void __launch_bounds__(256) gather_quant_mxfp8_kernel(MxQuantParams p) {
+// bytes in tcgen05.cp order.  A warp takes LOADS x 256 values of a row at a time, all of a lane's 16-byte loads in flight.
+// With a table the sort made (num_rows set) a CTA column works on one 128-row block: its routed rows come first, so their
+// count -- one look at the block's ids -- is all the work there is, plus zero codes for the padding rows that the GEMM's
+// producer loads.  (Walking every row of the table, padding included, took 65 us for 64 tokens on 231 experts, of which 576
+// rows of 29.6 k are routed.)  Rows in place order, or through a caller's table, are one run that all CTAs share.
+template <int LOADS, bool BLOCKS>
+__global__ void __launch_bounds__(256, LOADS == 1 ? 8 : 4) gather_quant_mxfp8_kernel(MxQuantParams p) {
   griddep_wait();
   griddep_launch();
   const int groups_per_row = p.hidden >> 5;
   const int KB = p.hidden >> 7;
-  const int n_rows = p.num_rows ? min(*p.num_rows, p.n_rows) : p.n_rows;
+  const int n_rows = BLOCKS ? min(*p.num_rows, p.n_rows) : p.n_rows;
   const int lane = threadIdx.x & 31, sub = threadIdx.x & 3;
   const uint32_t group_mask = 0xFu << (threadIdx.x & 28);
-  const int segments = (p.hidden + kMxQuantSegment - 1) / kMxQuantSegment;
-  const int first_item = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), item_step = gridDim.y * (blockDim.x >> 5);
-  for (int row0 = blockIdx.x * 128; row0 < n_rows; row0 += gridDim.x * 128) {
-    int live = min(128, n_rows - row0);
-    if (p.num_rows)  // a table the sort made; one that a caller made may hold its -1 rows anywhere
-      live = __syncthreads_count(threadIdx.x < live && p.sorted_ids[row0 + threadIdx.x] >= 0);
+  const int segments = (p.hidden + 256 * LOADS - 1) / (256 * LOADS);
+  const int part = BLOCKS ? blockIdx.y : blockIdx.x, parts = BLOCKS ? gridDim.y : gridDim.x;
+  const int first_item = part * (blockDim.x >> 5) + (threadIdx.x >> 5), item_step = parts * (blockDim.x >> 5);
+  for (int row0 = BLOCKS ? blockIdx.x * 128 : 0; row0 < n_rows; row0 += BLOCKS ? gridDim.x * 128 : n_rows) {
+    int live = n_rows - row0;
+    if (BLOCKS) live = __syncthreads_count(threadIdx.x < min(128, live) && p.sorted_ids[row0 + threadIdx.x] >= 0);
     for (int item = first_item; item < live * segments; item += item_step) {
-      const int row = row0 + item / segments;
-      const int c0 = item % segments * kMxQuantSegment + lane * 8;  // this lane's first value; the others 256 apart
+      const int r0 = static_cast<int>(static_cast<uint32_t>(item) / static_cast<uint32_t>(segments));
+      const int row = row0 + r0;
+      const int c0 = (item - r0 * segments) * (256 * LOADS) + lane * 8;  // this lane's first value; the others 256 apart
       const int rid = p.sorted_ids ? p.sorted_ids[row] : row;  // no table: quantise the rows in place order
       if (rid < 0) continue;
       const int token = rid / p.routes_per_token;
       const uint16_t* x = reinterpret_cast<const uint16_t*>(p.x) + static_cast<size_t>(token) * p.hidden;
-      uint4 raw[kMxQuantSegment / 256];
+      uint4 raw[LOADS];
 #pragma unroll
-      for (int u = 0; u < kMxQuantSegment / 256; ++u)
+      for (int u = 0; u < LOADS; ++u)
         if (c0 + u * 256 < p.hidden) raw[u] = *reinterpret_cast<const uint4*>(x + c0 + u * 256);
 #pragma unroll
-      for (int u = 0; u < kMxQuantSegment / 256; ++u) {
+      for (int u = 0; u < LOADS; ++u) {
         const int col = c0 + u * 256, grp = col >> 5;
         if (col >= p.hidden) continue;  // uniform over a group's four lanes: hidden is a multiple of 128
         const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(256) gather_quant_mxfp8_kernel(MxQuantParams p
         if (sub == 0) p.scales[scale_at] = static_cast<uint8_t>(ex + 127);
       }
     }
-    if (p.num_rows && p.zero_padding) {
+    if (BLOCKS && p.zero_padding) {
       const int loaded = p.zero_padding == 1 ? 128 : 16 << small_box_index(p.sorted_ids, row0);
       const int vec_per_row = p.hidden >> 4;
       uint4* z = reinterpret_cast<uint4*>(p.q + static_cast<size_t>(row0) * p.hidden);
@@ -777,6 +779,12 @@ __global__ void __launch_bounds__(256) gather_rows_mxfp8_kernel(MxQuantParams p)
 }  // namespace
 
 
+// Rows in place order or through a caller's table: four loads in flight per lane from this many values on, one below, where
+// the chip is not full and a lane's chain is all there is (150 x 7168, 1.1 M values, 2.9 / 2.3 us with four / one; 300 x 7168,
+// 2.2 M, 3.2 / 3.5; 8192 x 7168 34 / 44), by at most 8 CTAs per SM (8192 x 7168 33.2 / 33.6 / 37.9 us with 4 / 8 / no limit,
+// 8192 x 2048 11.4 / 10.3 / 11.0).  A CTA column per 128 rows, as for the sort's table, took 8.0 us at 150 and 300 x 7168.
+constexpr int64_t kMxWideFrom = int64_t{2} << 20;
+constexpr int kMxFlatCtas = 148 * 8;
 int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream) {
   if (p.hidden % 128 != 0) return AKLR_ERR_UNSUPPORTED_SHAPE;
   if ((p.q_lo != nullptr) != (p.scales_lo != nullptr) || (p.q_lo && (p.q_in || p.act_fp4))) return AKLR_ERR_BAD_ARGUMENT;
@@ -788,12 +796,20 @@ int launch_gather_quant_mxfp8(const MxQuantParams& p, cudaStream_t stream) {
     return launch_kernel(gather_rows_mxfp8_kernel, dim3(grid), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
   }
   if (static_cast<int64_t>(p.n_rows) * (p.hidden / 32) >= (int64_t{1} << 31)) return AKLR_ERR_TOO_LARGE;
+  if (!p.num_rows) {
+    const int loads = static_cast<int64_t>(p.n_rows) * p.hidden < kMxWideFrom ? 1 : 4;
+    const int64_t items = static_cast<int64_t>(p.n_rows) * ((p.hidden + 256 * loads - 1) / (256 * loads));
+    const int64_t ctas = (items + 7) / 8;
+    return launch_kernel(loads == 1 ? gather_quant_mxfp8_kernel<1, false> : gather_quant_mxfp8_kernel<4, false>,
+                         dim3(static_cast<unsigned>(ctas < kMxFlatCtas ? ctas : kMxFlatCtas)), dim3(256), 0, stream, 1, p) == cudaSuccess
+               ? AKLR_OK : AKLR_ERR_CUDA;
+  }
   // one CTA column per 128-row block; where the blocks are few, several CTAs share a block's rows
   const int64_t blocks = (static_cast<int64_t>(p.n_rows) + 127) / 128;
   const int grid = static_cast<int>(blocks < 65535 ? blocks : 65535);
   int share = 148 * 8 / grid;
   share = share < 1 ? 1 : share > 32 ? 32 : share;
-  return launch_kernel(gather_quant_mxfp8_kernel, dim3(grid, share), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
+  return launch_kernel(gather_quant_mxfp8_kernel<4, true>, dim3(grid, share), dim3(256), 0, stream, 1, p) == cudaSuccess ? AKLR_OK : AKLR_ERR_CUDA;
 }
 
 int grouped_gemm_mx_pick_stages(bool gate_up, bool split) {

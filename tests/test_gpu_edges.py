@@ -170,6 +170,39 @@ def test_quantised_codes_do_not_depend_on_the_outputs_alignment(rows, hidden):
     assert torch.equal(scales.cpu(), (amax.clamp_min(1e-10) * torch.tensor(1.0 / 448.0)).T.contiguous())
 
 
+@pytest.mark.parametrize("rows,hidden", [(1, 128), (63, 16384), (64, 16384), (65, 16384), (1100, 1024)])
+def test_quantised_rows_do_not_depend_on_the_rows_beside_them(rows, hidden):
+    """Sixteen lanes per group in launches below 8192 groups (63 rows of 16384 and less), eight from there: the same codes and
+    scales, bit for bit, for the same rows in a call of their own -- infinities, NaN, zeros, the largest and the smallest
+    values among them.  The MXFP8 quantiser of per-token rows changes its warps' share of a row with the call's size, too."""
+    from aklr_b200 import _lib
+    from aklr_b200.moe import act_quant_fp8, per_group_quant_fp8
+
+    def mx_rows(x):
+        codes = torch.empty(x.shape, dtype=torch.uint8, device=dev())
+        scales = torch.empty((x.shape[0], hidden // 32), dtype=torch.uint8, device=dev())
+        order = torch.arange(x.shape[0], dtype=torch.int32, device=dev())
+        stream = torch.cuda.current_stream().cuda_stream
+        _lib.check(_lib.load().aklr_ep_gather_quant_mxfp8(x.data_ptr(), order.data_ptr(), x.shape[0], hidden, 1,
+                                                          codes.data_ptr(), scales.data_ptr(), stream))
+        return codes, scales
+
+    x = torch.randn(rows, hidden, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16)
+    special = [float("inf"), float("-inf"), float("nan"), 0.0, torch.finfo(torch.bfloat16).max, 2.0**-126, 2.0**-133, -3.0e-30]
+    for i, value in enumerate(special[: hidden // 16]):
+        x[0, 16 * i] = value
+    x[rows - 1, :128] = 0.0
+    x = x.to(dev())
+    for quantise, by_group in ((act_quant_fp8, False), (per_group_quant_fp8, True), (mx_rows, False)):
+        codes, scales = quantise(x)
+        scales = scales.T if by_group else scales
+        for row in {0, rows // 2, rows - 1}:
+            alone, alone_scales = quantise(x[row : row + 1].contiguous())
+            alone_scales = alone_scales.T if by_group else alone_scales
+            assert torch.equal(alone.view(torch.uint8), codes[row : row + 1].view(torch.uint8)), quantise
+            assert torch.equal(alone_scales.contiguous().view(torch.uint8), scales[row : row + 1].contiguous().view(torch.uint8))
+
+
 @pytest.mark.parametrize("groups,limit", [(1, 256), (8, 1536)])
 def test_routing_is_the_same_on_both_sides_of_the_kernels_line(groups, limit):
     """256 experts, sigmoid: counted up to 256 tokens without groups and 1536 with them, warp arg-maxes past that.  The
