@@ -26,12 +26,11 @@ def router_case(tokens, hidden, experts, dtype):
 @pytest.mark.parametrize("tokens", [1, 2, 3, 16, 17, 63, 64, 129])
 @pytest.mark.parametrize("hidden,experts", [(136, 7), (192, 33), (2048, 512), (7168, 256)])
 def test_bf16_router_at_every_shape_of_its_kernels(tokens, hidden, experts):
-    """One token, 2 x 2 and 2 x 4 dot products per warp, the tensor-core tiles with one and two boxes of K per stage.
+    """One token, 2 x 2 and 2 x 4 dot products per warp (at 136 columns, no whole boxes of K, for every batch size), the
+    tensor-core tiles of 16 experts with one and two boxes of K per stage.
     Bound: the rounding to bf16 (2^-8 of the value) and at most 2^-23 of the sum of magnitudes for every 16th of the chain."""
     from aklr_b200.moe import router_logits
 
-    if hidden % 64 and tokens >= 64:
-        pytest.skip("the tensor-core kernel needs whole boxes of K: such a call takes the dot products tested below 64 tokens")
     x, w, exact, magnitude = router_case(tokens, hidden, experts, torch.bfloat16)
     got = router_logits(x.to(dev()), w.to(dev())).cpu().double()
     assert ((got - exact).abs() <= 2.0**-8 * exact.abs() + (hidden / 16 + 16) * 2.0**-23 * magnitude).all()
@@ -82,6 +81,37 @@ def test_float32_router_keeps_float32_accuracy(tokens, hidden, experts):
         assert ((again - exact).abs() <= (hidden + 32) * 2.0**-24 * magnitude).all()
 
 
+@pytest.mark.parametrize("tokens", [1, 16, 17, 300])
+def test_float32_router_refuses_widths_it_has_no_kernel_for(tokens):
+    from aklr_b200 import _lib
+    from aklr_b200.moe import router_logits_f32
+
+    x, w, _, _ = router_case(tokens, 192, 8, torch.float32)
+    with pytest.raises(_lib.AklrError) as err:
+        router_logits_f32(x.to(dev()), w.to(dev()))
+    assert err.value.code == -4  # AKLR_ERR_UNSUPPORTED_SHAPE: hidden is not a multiple of 128
+
+
+@pytest.mark.parametrize("tokens", [17, 128, 300])
+@pytest.mark.parametrize("hidden,experts", [(128, 33), (768, 40), (3072, 96), (7168, 257)])
+def test_float32_router_adds_every_term_exactly_once(tokens, hidden, experts):
+    """Weights 1 + m 2^-17, m < 1024: the first bf16 term is 1, the second holds m's leading eight bits and the third the
+    rest.  Activations +a, -a in pairs, the last pair of every 64 is +a, 0, so that every K step adds one to the first term's
+    sum.  Every partial sum of every term is a multiple of 2^-17 below 2^7 (times a), so float32 holds all of them exactly in
+    any order: a term, a K step or an accumulator left out or added twice shows in the bits, in each expert tile."""
+    from aklr_b200.moe import router_logits_f32
+
+    g = torch.Generator().manual_seed(hidden + tokens)
+    w = 1.0 + torch.randint(0, 1024, (experts, hidden), generator=g).double() * 2.0**-17
+    sign = torch.randint(0, 2, (tokens, hidden // 2, 1), generator=g).double() * 2 - 1
+    x = torch.cat([sign, -sign], dim=2)
+    x[:, 31::32, 0], x[:, 31::32, 1] = 1.0, 0.0
+    x = x.view(tokens, hidden) * 2.0 ** (torch.arange(tokens) % 3 - 1).double()[:, None]
+    exact = x @ w.T
+    got = router_logits_f32(x.to(torch.bfloat16).to(dev()), w.float().to(dev()))
+    assert torch.equal(got.cpu().double(), exact)
+
+
 @pytest.mark.parametrize("tokens", [1, 16, 17, 130])
 @pytest.mark.parametrize("experts", [33, 256])
 def test_router_infinities_do_not_depend_on_the_batch_size(tokens, experts):
@@ -130,18 +160,23 @@ def test_sort_with_and_without_the_per_warp_counts(n_experts, n_tokens, k, block
 @pytest.mark.parametrize("copies", [1, 3])
 def test_mxfp4_boxes_at_their_edges(inter, act_bits, copies):
     """Experts with 1, 8, 9, 16, 17, ... routed rows (boxes of 16, 32, 64 and 128 rows, direct and staged output rows, warps
-    without a row): bit for bit the output of loading all 128 rows, and the oracle's within its gates.  Three routes per
-    token and more than 512 tokens: quantised once per token, then copied."""
+    without a row): bit for bit the output of loading all 128 rows, and the oracle's within its gates.  With three routes per
+    token and more than 512 tokens the same rows are quantised once per token, then copied."""
     from aklr_b200 import _lib
     from aklr_b200.moe import fused_experts_mxfp4
 
     rows = [1, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129]
-    cfg = wl.MoEConfig("mx", hidden=256, inter=inter, n_routed=len(rows) + 1, topk=1)
+    fillers = 4  # experts after them that take the other routes of a token with three
+    cfg = wl.MoEConfig("mx", hidden=256, inter=inter, n_routed=len(rows) + fillers + 1, topk=copies)
     weights = [t.to(dev()) for t in wl.mx_expert_weights(cfg, 5)]
     ids = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(rows)])  # the last expert gets none
     g = torch.Generator().manual_seed(inter + act_bits)
     ids = ids[torch.randperm(ids.numel(), generator=g)].view(-1, 1)
-    ids = torch.cat([(ids + 5 * c) % len(rows) for c in range(copies)], dim=1).contiguous()
+    if copies == 3:  # one route to an edge-sized expert in a random slot, two to the fillers
+        t = torch.arange(ids.shape[0], dtype=torch.int32).view(-1, 1)
+        ids = torch.cat([ids, len(rows) + t % 2, len(rows) + 2 + t % 2], dim=1)
+        ids = ids.gather(1, torch.rand(ids.shape, generator=g).argsort(1)).contiguous()
+    assert torch.bincount(ids.flatten(), minlength=cfg.n_routed)[: len(rows)].tolist() == rows
     x = torch.randn(ids.shape[0], 256, generator=g).to(torch.bfloat16)
     route_weights = torch.rand(ids.shape, generator=g)
     outs = []
