@@ -16,8 +16,9 @@ namespace aklr {
 
 // A warp takes ``chunks_per_item`` runs of 256 columns of one token: its routes are looked at once per item, one lane
 // each, and are a bit mask from then on, so that a thread is left with its rows' loads (nine at a time in flight) and
-// additions.  With every thread reading and testing all of its token's ids per 8 columns the pass issued 45 % of its cycles
-// at three CTAs per SM and reached 69 % of the memory's rate (16384 tokens x 9 routes on 7168, 2.35 GB: 490 -> 385 us, 6.1 TB/s).
+// additions.  With every thread reading and testing all of its token's ids per 8 columns, 16384 tokens x 9 routes on 7168
+// (2.35 GB) took 490 us, 4.8 TB/s; so 385, 6.1.  (In a capture at 4096 tokens that form issued in 45 % of its cycles at three
+// CTAs per SM and used 69 % of the memory's nominal rate, this one 75 %.)
 constexpr int kCombineSlots = 9;
 __global__ void __launch_bounds__(256, 4) combine_kernel(CombineParams p, int chunks_per_item, int items_per_token) {
   griddep_wait();
@@ -282,7 +283,7 @@ int launch_add_gated_rows(const void* x, const void* gate, const void* rows, voi
 // rounded).  CUDA cores, float32 FMAs in k order.
 //  * few tokens: one warp per (token, expert) dot product, so the weight is read by many SMs;
 //  * else the tensor cores (router_gemm.cu); this file keeps a 64 x 64 tile per CTA, 16 k per step, 4 x 4 outputs per
-//    thread, for token rows a TMA load cannot start at.
+//    thread, for token rows a TMA load cannot start at and logits that 16-byte stores cannot (off a 16-byte boundary).
 template <int UNROLL>  // strides whose loads are in flight together (see router_gemm_kernel)
 __global__ void __launch_bounds__(256)
 router_dot_f32_kernel(const uint16_t* __restrict__ x, const float* __restrict__ w, float* __restrict__ logits,

@@ -20,8 +20,10 @@
 //
 // Outcome on B200 (DeepSeek-V3 widths, 4096 / 16384 tokens): bit-identical outputs, gate_up 2.8 / 8.3 ms against
 // 2.0 / 5.9 ms of the two-buffer kernel.  Twice the K-blocks, each with the same fixed cost: the waits on
-// free TMEM buffers are gone, the period per K-block is not.  It is therefore NOT the default; a call selects
-// it with AKLR_VARIANT_DEEP_PIPELINE, and it stays in the test suite as the measurement of "more buffers".
+// free TMEM buffers are gone, the period per K-block is not.  Part of that cost is how the MMAs are issued here: by
+// one lane under lane == 0, 433 cycles for four N=128 MMAs that take the pipe 256, where elect.sync (the other GEMM kernels'
+// way) would take about 130.  So this does not say what four buffers are worth with cheap issue; that has not been
+// measured.  It is NOT the default; a call selects it with AKLR_VARIANT_DEEP_PIPELINE.
 //
 // Warp roles (384 threads): warp 0 TMA producer, warps 1-2 MMA issuers taking K-blocks alternately (warp 1
 // owns TMEM), warp 3 idle, warps 4-11 epilogue (TMEM lane quarter = warp % 4, column half = (warp-4)/4);

@@ -54,8 +54,10 @@ struct MxLayout {
 
 constexpr int kOutPassCols = 32;  // down: channels per thread staged per pass (64 bytes per row)
 // down: a warp with at most this many routed rows stores them from registers.  Staging pays where the lanes store to 32
-// different rows; it is four times the same chain of shared-memory round trips whatever the number of rows.  64 tokens on 231
-// experts (2.5 rows a block): 227.1 -> 200.6 us for the layer.
+// different rows; it is four times the same chain of shared-memory round trips whatever the number of rows.  The layer on
+// 6144 x 256, 257 experts, top 9, with the line at 0 / 8 / 16 / 32 rows, microseconds: 64 tokens (2.3 rows a block) 194 / 184 /
+// 184 / 184; 256 tokens (9 rows) 220 / 214 / 209 / 208; 511 (18) 239 / 239 / 236 / 231; 1024 (36) 275 / 272 / 272 / 281; 2048
+// (72) 349 / 348 / 348 / 496; 4096 595 / 594 / 597 / 895.  So the line is safe anywhere up to 16.
 constexpr int kDirectRows = 8;
 
 __host__ __device__ inline MxLayout mx_layout(int stages, bool gate_up, bool split) {

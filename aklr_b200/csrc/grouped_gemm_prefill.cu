@@ -19,19 +19,18 @@
 // warpgroup gives its registers to the epilogue (setmaxnreg 40 / 232): 128 accumulators + 64
 // staging registers per epilogue thread do not fit the 168 an even split allows.
 //
-// What bounds it, measured on B200 piece by piece on all 148 SMs: the four MMAs of a K-block take 512 cycles
-// with nothing else running (nominal) and 665-750 next to the fold; the fold alone 333-364 (8 tcgen05.ld x32
-// per warp + 128 packed FMAs per thread); a TMA ring alone delivers 48 KB per ~520 cycles; the kernel's
-// period is 1100-1450.  No piece explains it: the hand-offs of the MMA <-> fold cycle each arrive late (512
-// TMEM columns hold exactly two N=256 partials, and a ring stage is held until the MMAs that read it are
-// done).  What helped: one commit per K-block and a lean MMA-issue loop, scales prefetched from global
-// memory two K-blocks ahead instead of staged per tile, register hand-over (setmaxnreg).  What did not: weight
-// tiles prefetched into L2 ahead of the ring (+1-3% at 4096 tokens, -18% at 1024 where every tile's weights
-// come from HBM), per-half hand-offs (two N=128 MMA groups; 20%
-// slower), 128 x 128 tiles with four partials in flight (grouped_gemm_deep.cu; 40% slower), two MMA-issuing
-// threads, one polling lane per warp, issuing the next K-block's first batch early, 16 epilogue warps,
-// larger or single-buffered load batches, CTA pairs (below).  Persistent CTAs, TMA SWIZZLE_128B ring,
-// two 256-column TMEM partial buffers, no multicast loads, bounded waits.
+// What bounds it is the epilogue.  Counters inside a copy of it, cycles per K-block at 4096 tokens: period 1197; the MMA
+// warp waits 133 for operands, 693 for a free TMEM buffer and issues for 246; an epilogue warp waits 157 for its partial,
+// loads and folds for 657, and spends the other ~380 on its scales and on the starts and ends of tiles.  Alone, on all 148
+// SMs: the four MMAs of a K-block 512 cycles (nominal; 665-750 next to the fold), the fold 333-364 (8 tcgen05.ld x32 per warp
+// + 128 packed FMAs per thread), a TMA ring 48 KB per ~520.  What helped: one commit per K-block and a lean MMA-issue
+// loop under elect.sync, scales prefetched from global memory two K-blocks ahead instead of staged per tile, register
+// hand-over (setmaxnreg).  What did not: weight tiles prefetched into L2 ahead of the ring (+1-3% at 4096 tokens, -18% at
+// 1024 where every tile's weights come from HBM), per-half hand-offs (two N=128 MMA groups, 7-16% slower under elect.sync),
+// two MMA-issuing threads, one polling lane per warp, issuing the next K-block's first batch early, 16 epilogue
+// warps, larger or single-buffered load batches, CTA pairs (below).  128 x 128 tiles with four partials in flight
+// (grouped_gemm_deep.cu) are slower too, as far as that has been measured: with their MMAs issued under lane == 0.
+// Persistent CTAs, TMA SWIZZLE_128B ring, two 256-column TMEM partial buffers, no multicast loads, bounded waits.
 #include <cfloat>
 #include <map>
 #include <mutex>

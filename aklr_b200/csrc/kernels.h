@@ -245,9 +245,11 @@ struct EpCombineParams {
 };
 int launch_ep_combine(const EpCombineParams& p, cudaStream_t stream);
 
-// tensor-core router GEMM (router_gemm.cu): maps are bf16 [T,H] box 64 x 128 and [E,H] box 64 x n_tile
+// tensor-core router GEMMs (router_gemm.cu); map_x is bf16 [T,H] with boxes of 64 x 128.
+// float32 weights: map_w is float32 [E,H], boxes of 64 x 32
 int launch_router_gemm_f32_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, float* logits, int n_tokens, int hidden,
                               int n_routed, int32_t* host_status, cudaStream_t stream);
+// bf16 weights: map_w is bf16 [E,H], boxes of 64 x n_tile
 int router_gemm_tc_pick_n_tile(int n_tokens, int n_routed, int sm_count);
 int launch_router_gemm_tc(const CUtensorMap& map_x, const CUtensorMap& map_w, void* logits, int n_tokens, int hidden,
                           int n_routed, int n_tile, int32_t* host_status, cudaStream_t stream);

@@ -1,6 +1,7 @@
 // Does a TMA ring writing shared memory slow the tensor core's reads of it?  148 CTAs; each runs
 // (a) an MMA stream on a fixed operand pair in shared memory (M128 N256 K128 e4m3 per "K-block", two deep),
 // (b) a TMA ring of 48 KB stages into OTHER shared memory, recycled at once,  alone and together.
+// (One lane issues under lane == 0; the product kernels issue under elect.sync, at a third of the issue cost.)
 #include <cstdio>
 #include <cstdlib>
 #include <cuda.h>

@@ -1,5 +1,6 @@
 // What an issuing thread pays per tcgen05.mma and how far the tensor pipe lets it run ahead: bursts of n MMAs (M128, N256, K32)
 // from an idle pipe, cycles until the issue loop returns and until the commit of the burst is seen.
+// One lane issues under lane == 0, which costs it ~100 cycles per MMA; the product kernels issue under elect.sync (common.cuh), ~30.
 #include <cstdio>
 #include "../common.cuh"
 using namespace aklr;

@@ -1,5 +1,6 @@
 // Tensor-pipe timing of tcgen05.mma kind::f8f6f4 (M128, K32): cycles per MMA as a function of N and of how
 // many INDEPENDENT accumulators the issuing thread rotates over (1 = every MMA depends on the one before).
+// (One lane issues under lane == 0; the product kernels issue under elect.sync, at a third of the issue cost.)
 #include <cstdio>
 #include "../common.cuh"
 using namespace aklr;

@@ -2,6 +2,7 @@
 // (M128, N256, K32, one issuing thread per SM, all 148 SMs) on constant operands (every byte e4m3 1.0) and on
 // random bytes, short (4096 MMAs, 0.3 ms) and long (65536 MMAs, several ms): cycles per MMA from clock64,
 // nanoseconds per MMA from the global timer, and the SM clock the two imply.
+// (One lane issues under lane == 0; the product kernels issue under elect.sync, at a third of the issue cost.)
 #include <cstdio>
 #include "../common.cuh"
 using namespace aklr;

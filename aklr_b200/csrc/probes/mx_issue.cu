@@ -1,6 +1,7 @@
 // Issue stream of the MXFP4 grouped GEMM alone: per K-block the thread copies scale factors into TMEM with
 // tcgen05.cp (0..4 copies) and issues four kind::mxf8f6f4.block_scale MMAs (M 128, N 256, K 32) on one accumulator.
 // Cycles per K-block as a function of the number of copies, and with the copies writing alternating column sets.
+// (One lane issues under lane == 0; the product kernels issue under elect.sync, at a third of the issue cost.)
 #include <cstdio>
 #include "../common.cuh"
 using namespace aklr;

@@ -188,17 +188,18 @@ __global__ void __launch_bounds__(kThreads, 1) router_gemm_tc_kernel(const __gri
 // ---- float32 router weights ----------------------------------------------------------------------
 // logits[T, E] = x[T, H] (bf16) . W[E, H]^T (float32), float32 logits, nothing rounded on the way in: a float32 weight
 // is the sum of three bf16 terms (its 24 significant bits cut into 8 + 8 + 8, exact short of underflow), a product of two
-// bf16 values is exact in float32, and the three products' sums are kept apart and added once, smallest first.  So the only roundings are those of the accumulation, 1/12th as many per element as a
-// CUDA-core chain over H has (K = 16 per MMA), in kF32Slices accumulators of the first term that share K out between them.
+// bf16 values is exact in float32, and the three products' sums are kept apart and added once, smallest first.  So the
+// only roundings are those of the accumulation: one per 16 products (K = 16 per MMA), in kF32Slices accumulators of the first
+// term that share K out between them, where a CUDA-core chain over H has one per product.
 // An infinite activation times a low term that is zero is NaN where the product itself is infinite, so a logit whose first
 // term is not finite is that term's sum alone: +-inf and NaN come out as from the CUDA-core kernels, whatever the batch
 // size.  (The first term of a weight below 2^-133 is zero too: its product with an infinity is NaN here.)
 //
 // One CTA per 128 tokens x 32 experts, 64 of K per stage: TMA loads the bf16 token tile (16 KB, SWIZZLE_128B) and the
-// raw weights (32 x 64 floats), four warps turn the weights into one 96-row operand tile (32 rows of each term, swizzled
-// as the MMA reads it), and two MMAs of M128 K16 per step cover the first term (N 32) and the other two (N 64).  320
-// threads: warp 0 TMA, warp 1 MMA + TMEM, warps 2..9 conversion on alternate stages,
-// warps 2..5 then the epilogue.  2000 tokens on 3072 x 256: 194 us on the CUDA cores (bound by shared-memory
+// raw weights (32 x 64 floats), four of eight warps turn the weights into one 96-row operand tile (32 rows of each term,
+// swizzled as the MMA reads it), and two MMAs of M128 K16 per step cover the first term (N 32) and the other two (N 64).
+// 320 threads: warp 0 TMA, warp 1 MMA + TMEM, warps 2..5 and 6..9 conversion of alternate stages, warps 2..5 then the
+// epilogue.  2000 tokens on 3072 x 256: 194 us on the CUDA cores (bound by shared-memory
 // reads of a 4 x 4 tile per thread and a memory round trip per 16 k), 30 us here; against 64 bits the relative error (2-norm) fell from 9.9e-7 to 2.4e-7, at
 // 4096 x 7168 from 1.5e-6 to 5.8e-7 (with 4 accumulators it would be 1.8e-6: the MMA truncates as it accumulates).
 constexpr int kF32Experts = 32;

@@ -328,8 +328,10 @@ __global__ void __launch_bounds__(1024) route_count_kernel(RouteParams p) {
 // Whether a batch is routed by counting (one CTA per token) or by warp arg-maxes.  A count compares every key with every
 // other of its group: short for grouped routing, E * E per token without groups.  Microseconds per launch, counting / warps,
 // at 64, 512 and 2048 tokens: grouped 256 experts 3.1 / 9.7, 5.9 / 10.0, 13.6 / 12.8; sigmoid 256 experts without groups
-// 4.3 / 5.9, 9.7 / 6.1, 28.7 / 7.2 (equal at 256 tokens); softmax, whose scores need no work before they are ranked, 128
-// experts 2.6 / 2.1, 3.9 / 2.2, 9.2 / 2.7, 512 experts 9.1 / 6.9, 30.4 / 7.2, 102 / 9.3, 8 experts 1.7 / 1.5, 1.7 / 1.6, 3.0 / 1.8.
+// 4.3 / 5.9, 9.7 / 6.1, 28.7 / 7.2 (equal at 256 tokens; with 1024 experts 29.5 / 20.1 at 128); softmax, whose scores need no
+// work before they are ranked, 128 experts 2.6 / 2.1, 3.9 / 2.2, 9.2 / 2.7, 512 experts 9.1 / 6.9, 30.4 / 7.2, 102 / 9.3, 8
+// experts 1.7 / 1.5, 1.7 / 1.6, 3.0 / 1.8, and at one and 16 tokens 8 experts 1.5 / 1.4, 1.6 / 1.4, 60 experts 1.9 / 1.5, 2.0 / 1.6,
+// 512 experts 9.0 / 6.2, 9.0 / 7.0, 1024 experts 29.0 / 10.9, 29.2 / 11.8: the warps at every size.
 static bool routes_by_counting(const RouteParams& p) {
   if (p.num_expert_group > 1 && p.topk_group < p.num_expert_group) return p.n_tokens <= 1536;
   return p.scoring == AKLR_SCORING_SIGMOID && static_cast<int64_t>(p.n_tokens) * p.n_routed <= 256 * 256;
@@ -506,8 +508,9 @@ __device__ void plan_blocks(const AlignParams& p, const int* total, int* base, i
 // ``warp_counts`` [32][n_experts] (smem): how many routes of the chunk each warp has for each expert; one thread per
 // expert then sums over the warps, and the chunk takes four barriers.  Without the table -- null, where the expert counts do
 // not fit, and chunks of at most kSerialWarps warps -- the warps take their rows one after the other, a barrier each:
-// 333 tokens x 8 routes, three chunks in one CTA, 19.6 us that way, 13.2 by the table; 17 tokens x 11 routes (six warps, 513
-// experts) 83.1 us for the call that way, 86.4 by the table.
+// 333 tokens x 8 routes, three chunks in one CTA, 19.6 us that way, 13.2 by the table.  Where the line lies matters little
+// between three and nine warps: the sort alone is 0.1-0.4 us faster by the table there (257 experts, 3 / 5 / 7 warps 3.83 / 4.31 /
+// 4.87 by turns, 3.62 / 3.98 / 4.46), a layer call 0-0.4 us (8 to 24 tokens on 257 and 513 experts); one and two warps are level.
 constexpr int kSerialWarps = 8;
 constexpr int kWarpCountExperts = 544;  // 32 x 544 counts and the int arrays stay under the 48 KB a launch gets unasked
 __device__ void place_chunk(const AlignParams& p, int route, int* cursor, uint16_t* warp_counts) {
